@@ -656,14 +656,8 @@ def survey_arm(args, rank, local_rank, world, dist):
     return line
 
 
-# Grid bytes one in-box RK4 step gathers per time level read: 4 RHS x 8
-# corners x 40 Gamma x 4 bytes (5 aligned 32-byte loads per corner).
-GATHER_BYTES_PER_LEVEL = 4 * 8 * 40 * 4
-PEAK_L1_GATHER = 2  # GRAY_PEAK_L1_GATHER of include/gray_cuda.h
-
-
 def gather_levels(cfg, grid_t1, physics):
-    """Time levels a gather reads.  In physics mode the time factor is
+    """Time levels a step in the box reads.  In physics mode the time factor is
     clamped to [0, 1] and a level of zero weight is not fetched, so a render
     traced backward from the first level's time reads that level alone."""
     if physics and cfg["t_init"] <= grid_t1 and cfg["dt_dump"] < 0:
@@ -674,10 +668,11 @@ def gather_levels(cfg, grid_t1, physics):
 def numerical_arm(args, cfg, rank, local_rank, world, dist):
     """numerical_128: boosted-KS 128^3 grid with two time levels (t = 0,
     10 M) over [-40, 40]^3, 512^2 camera at 200 M, mixed precision, physics
-    mode (flat outside the box).  The kernel is gather-bound: roofline in
-    algorithmic gather bytes (40 Gamma x 8 corners x 2 levels x 4 RHS per
-    in-box step and level read) against the L1 bandwidth of the same gather
-    pattern, measured in the run; DRAM traffic is reported beside it."""
+    mode (flat outside the box).  The kernel holds each ray's cell in
+    registers, so its in-box steps are bound by the FP32 pipe: roofline in
+    their operations (the contraction of 40 Gamma at 8 corners per RHS and
+    level read) against the FMA peak measured in the run; DRAM traffic is
+    reported beside it."""
     import torch
     from gray_b200 import api
 
@@ -731,15 +726,14 @@ def numerical_arm(args, cfg, rank, local_rank, world, dist):
         with open(MEASURED_PEAKS) as f:
             hbm, hbm_src = json.load(f)["hbm_gbs"], "MEASURED_PEAKS.json hbm_gbs (measured)"
     levels = gather_levels(cfg, G["t1"], True)
-    per_step = GATHER_BYTES_PER_LEVEL * levels
-    achieved = gsteps * per_step / (ker / args.steps) / 1e9
-    l1 = ctx.measure_peak(PEAK_L1_GATHER) / 1e9
+    per_step = flops.numerical_per_step(levels)
+    achieved = gsteps * per_step / (ker / args.steps) / 1e12
+    peak32 = ctx.measure_peak(api.PREC_MIXED)
     traffic = None if args.side else TRAFFIC.get(args.workload)
-    roofline = {"bound": "l1", "achieved": achieved, "peak": l1, "unit": "GB/s",
-                "frac": achieved / l1, "traffic": traffic,
-                "peak_source": "L1 load microbenchmark in this run (32-byte loads, all hits, "
-                               "full lines)",
-                "bytes_per_gather_step": per_step, "levels_read": levels,
+    roofline = {"bound": "fp32", "achieved": achieved, "peak": peak32 / 1e12,
+                "unit": "TFLOP/s", "frac": achieved / (peak32 / 1e12), "traffic": traffic,
+                "peak_source": "FP32 FMA microbenchmark in this run",
+                "flops_per_gather_step": per_step, "levels_read": levels,
                 "hbm": {"dram_bytes_per_launch": traffic, "peak": hbm, "peak_source": hbm_src,
                         "frac": (traffic / (ker / args.steps) / 1e9 / hbm) if traffic else None},
                 "kernel": "dyst_mixed_kernel"}

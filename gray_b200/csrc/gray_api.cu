@@ -544,7 +544,8 @@ run_mixed(gray_ctx *c, Render *r, double t_init, double dt_dump, long long n_dum
 		if(!grid_ready(c))
 			return GRAY_ESTATE;
 		CK(launch_dyst_mixed_table(T, c->grid->gp, r->p.n_freq, r->d_queue, r->d_steps,
-		                           c->stream, c->mixed, r->d_steps + 1));
+		                           c->stream, c->mixed, dyst_between(c->grid->gp, &m, 1),
+		                           r->d_steps + 1));
 	} else {
 		CK(launch_mixed_table(T, r->p.n_freq, r->d_queue, r->d_steps, c->stream, c->mixed, &m));
 	}
@@ -1217,7 +1218,9 @@ batch_enqueue(gray_ctx *c, Batch *b, const MixedLaunch &cfg, const MixedTable &T
 	CK(cudaMemsetAsync(b->d_steps, 0, sizeof(unsigned long long), c->stream));
 	if(b->spacetime == GRAY_ST_NUMERICAL)
 		CK(launch_dyst_mixed_table(T, c->grid->gp, b->n_freq, b->d_queue, b->d_steps,
-		                           c->stream, cfg));
+		                           c->stream, cfg,
+		                           dyst_between(c->grid->gp, b->host_table.data(),
+		                                        (int)b->host_table.size())));
 	else
 		CK(launch_mixed_table(T, b->n_freq, b->d_queue, b->d_steps, c->stream, cfg, one));
 	return GRAY_OK;

@@ -1,26 +1,47 @@
 /*
  * Mixed-precision persistent kernel for numerical spacetimes (interp.cl +
- * dyst.cl): warp-refilled rays, FP32 gathers of the 40 Christoffel symbols
- * accumulated with packed f32x2 FMA over component pairs, compensated
- * (hi, lo) state update, FP64 null-constraint check at the end.
+ * dyst.cl): several lanes per ray, the ray's cell held in registers.
+ *
+ * A ray moves about 0.01 M per stage through cells 0.2-2 M wide, so the same
+ * 8 corners serve dozens to hundreds of RHS evaluations.  Lane m of a ray's
+ * four lanes owns x^m, u^m and row m of the Christoffel symbols: the ten
+ * Gamma^m_ab of the cell's 8 corners stay in 80 of its registers and are
+ * read from memory only when the ray enters another cell.  An RHS is then 40
+ * packed FMAs per lane (two corners each) and about ten shuffles, with no
+ * loads.  With one ray per thread the 40 symbols of 8 corners (320 floats)
+ * fit no thread, so every RHS fetched 1,280 bytes per ray through L1, and
+ * that latency bound the kernel.
+ *
+ * What bounds it: the FP32 pipe and issue, about evenly (FMA pipe 56% of its
+ * cycles, issue 63%, 158 instructions per warp and RHS against 105 counted
+ * from the algorithm; 12 warps per SM at 168 registers).  Measured, B200 at
+ * 1965 MHz, one ray per thread before and four lanes now: 512^2 rays at 200 M
+ * on a 128^3 grid 530 -> 197 ms (1.48e10 -> 3.99e10 ray-steps/s), 97 x 72
+ * rays on a 256^3 grid 243 -> 22.8 ms, 160 x 120 rays between two levels
+ * with four frequencies 44.6 -> 17.8 ms; outputs bit-identical.  The pairs
+ * are kept as 64-bit values: as float2 the compiler repacked the cell at
+ * every RHS (247 instructions, 301 ms).  At 128 registers and 16 warps the
+ * large render took 196 ms but the spills cost small ones 17% (20.3 ms
+ * against 17.3 at 64^2 rays).
+ *
+ * Where rays run between the two time levels (LV = 2) a ray has eight lanes,
+ * four per level.
+ *
+ * Thermal transfer: lanes 0 and 3 also hold their rows of g (for k_t and
+ * k_z), lane 1 rho, and the frequencies are divided among the ray's lanes.
  *
  * Grid layout: per time level float [nz][ny][nx][GRAY_NSTRIDE] with the
- * fields of one grid point contiguous (Gamma 0..39, g 40..49, rho 50, pad),
- * so the 8 corners of a cell are 8 rows of 224 bytes and the 40 Gamma of a
- * corner are 5 aligned 32-byte loads (sm_100 ld.global.v8.f32).  The fisheye node coordinates come
- * from a per-axis table (n + 1 entries) instead of sinh((A i + B)^3) per
- * field and call (interp.cl:99-121), and the cell search runs once per RHS
- * for all fields instead of once per field (102 times in the reference).
+ * fields of one grid point contiguous (Gamma 0..39, g 40..49, rho 50, pad).
+ * The fisheye node coordinates come from a per-axis table (n + 1 entries)
+ * instead of sinh((A i + B)^3) per field and call (interp.cl:99-121), and the
+ * cell search runs once per RHS for all fields instead of once per field
+ * (102 times in the reference).
  */
 #include <cfloat>
 #include <climits>
 
 #include "dyst64.cuh"
 #include "mixed_table.h"
-
-#ifndef GRAY_DYST_PREFETCH
-#define GRAY_DYST_PREFETCH 0
-#endif
 
 namespace {
 
@@ -65,24 +86,14 @@ struct DystConst {
 	float B[3], iA[3];
 };
 
-/* threads per block at most (the kernels' launch bound): the stride of the
- * per-thread cell cache in shared memory */
-constexpr int CELL_STRIDE = 256;
-
 /* Fractional logical coordinate on a fisheye axis, with the cell found
  * exactly against the node table: the FP32 map only gives the first guess,
  * node comparisons settle it (the answer depends on x and the table alone).
- * The last interior cell of each thread is kept in `cache` (x0, x1,
- * 1/(x1 - x0), i): a ray moves about 0.01 M per stage through cells 0.2-2 M
- * wide, so nearly every call skips the map (three MUFU in a chain) and the
- * two node loads, with the same result the search would give. */
+ * cell: an interior cell's x0, x1, 1/(x1 - x0), i; x0 > x1 outside. */
 __device__ __forceinline__ float
-axis_uvw32c(const GridParams &g, int a, float x, float Bf, float iAf, float4 &cache)
+axis_search(const float *nd, int n, float x, float Bf, float iAf, float4 &cell)
 {
-	if(x >= cache.x && x < cache.y)
-		return cache.w + (x - cache.x) * cache.z;
-	const int n = a == 0 ? g.nx : a == 1 ? g.ny : g.nz;
-	const float *nd = g.nodes_f[a];
+	cell = make_float4(INFINITY, -INFINITY, 0.0f, 0.0f);
 	if(!(x >= __ldg(nd)))
 		return 0.0f;              /* before the first node (or NaN): clamp-to-edge */
 	if(x >= __ldg(nd + n - 1))
@@ -106,25 +117,8 @@ axis_uvw32c(const GridParams &g, int a, float x, float Bf, float iAf, float4 &ca
 		x1 = __ldg(nd + i + 1);
 	}
 	const float inv = rcp_a(x1 - x0);
-	cache = make_float4(x0, x1, inv, (float)i);
-	return (float)i + (x - x0) * inv;
-}
-
-/* eight consecutive floats from a 32-byte aligned address, through the
- * read-only path */
-struct F8 {
-	float v[8];
-};
-
-__device__ __forceinline__ F8
-ldg8(const float *p)
-{
-	F8 r;
-	asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-	    : "=f"(r.v[0]), "=f"(r.v[1]), "=f"(r.v[2]), "=f"(r.v[3]), "=f"(r.v[4]), "=f"(r.v[5]),
-	      "=f"(r.v[6]), "=f"(r.v[7])
-	    : "l"(p));
-	return r;
+	cell = make_float4(x0, x1, inv, (float)i);
+	return fmaf(x - x0, inv, (float)i);
 }
 
 /* ------------------------------------------------ thermal transfer island */
@@ -149,15 +143,16 @@ exp_f(float x)
  * stay FP64, the special functions of O(1) arguments (exp, log, cbrt,
  * sqrt) take the FP32 approximate instructions, and everything that
  * depends only on the render is a ThermalFast constant.  Same formulas and
- * branches as the FP64 kernels; agreement to ~1e-6 relative. */
-template <int NF>
+ * branches as the FP64 kernels; agreement to ~1e-6 relative.  N: the
+ * frequencies of this lane. */
+template <int N>
 __device__ __forceinline__ void
-rt_rhs_fast(const ThermalFast &t, const double *nu_hz, const double *k, double ne,
+rt_rhs_fast(const ThermalFast &t, const double *nu_hz, double kt, double kz, double ne,
             const double *tau, double *dI, double *dtau)
 {
 	const double EPS = GRAY_EPSILON;
-	const double shift = -k[0];
-	const float bkcos = (float)(k[3] * t.b) * rcp_a((float)(shift * t.b + EPS));
+	const double shift = -kt;
+	const float bkcos = (float)(kz * t.b) * rcp_a((float)(shift * t.b + EPS));
 	const double ish2 = rcp64(fma(shift, shift, EPS));
 	/* synchrotron frequency: nu_s = knus sin(theta), zero along the field */
 	double nus = 0.0, inus = 0.0;
@@ -168,7 +163,7 @@ rt_rhs_fast(const ThermalFast &t, const double *nu_hz, const double *k, double n
 	}
 	const double ne2 = ne * ne;
 #pragma unroll
-	for(int i = 0; i < NF; ++i) {
+	for(int i = 0; i < N; ++i) {
 		const double nu = nu_hz[i] * shift;
 		/* rt.cl:80-93 */
 		const double f2 = nu * t.kf2;
@@ -223,588 +218,748 @@ rt_rhs_fast(const ThermalFast &t, const double *nu_hz, const double *k, double n
 	}
 }
 
-__device__ __forceinline__ bool
-inside32(const GridParams &g, const float *q)
+/* ------------------------------------------------------------ the kernel */
+
+/* The cell a lane holds: rows of ten (of Gamma^m_ab, a <= b) and, with the
+ * transfer, four more (row m of g, or rho), as pairs of corners (c, c + 1)
+ * along x, so that one packed FMA serves two corners. */
+typedef unsigned long long pair_t; /* two FP32 in one 64-bit register pair */
+
+__device__ __forceinline__ pair_t
+pair(float a, float b)
 {
+	pair_t r;
+	asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+	return r;
+}
+
+__device__ __forceinline__ float2
+unpair(pair_t a)
+{
+	float2 r;
+	asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+	return r;
+}
+
+__device__ __forceinline__ pair_t
+fma2(pair_t a, pair_t b, pair_t c)
+{
+	pair_t r;
+	asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+	return r;
+}
+
+__device__ __forceinline__ pair_t
+mul2(pair_t a, pair_t b)
+{
+	pair_t r;
+	asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+	return r;
+}
+
+template <bool RT>
+struct Cell {
+	pair_t G[4][10];
+	pair_t W[RT ? 4 : 1][RT ? 4 : 1];
+};
+
+/* the fields of lane m's extra row: row m of g (dyst.cl:55-81; g_zz from
+ * g_yz where the flag says so, dyst.cl:78) on lanes 0 and 3, rho on lane 1 */
+__device__ __forceinline__ int
+extra_field(int m, int k, int bug_gzz)
+{
+	if(m == 0)
+		return 40 + k;
+	if(m == 1)
+		return k == 0 ? 50 : -1;
+	if(m == 3)
+		return k == 0 ? 43 : k == 1 ? 46 : k == 2 ? 48 : bug_gzz ? 48 : 49;
+	return -1;
+}
+
+template <bool RT>
+__device__ __forceinline__ void
+load_cell(const GridParams &g, const float *lvl, int m, int ix, int iy, int iz, Cell<RT> &C)
+{
+	const int jx = min(ix + 1, g.nx - 1), jy = min(iy + 1, g.ny - 1), jz = min(iz + 1, g.nz - 1);
 #pragma unroll
-	for(int a = 1; a <= 3; ++a)
-		if(!(q[a] >= g.box[a] && q[a] <= g.box[a + 4]))
-			return false;
+	for(int j = 0; j < 4; ++j) {
+		const long long yz = (long long)((j & 2) ? jz : iz) * g.ny + ((j & 1) ? jy : iy);
+		const float *a = lvl + (yz * g.nx + ix) * GRAY_NSTRIDE;
+		const float *b = lvl + (yz * g.nx + jx) * GRAY_NSTRIDE;
+		/* 10 m floats into a 224-byte row: 8-byte aligned */
+		const float2 *ga = (const float2 *)(a + 10 * m), *gb = (const float2 *)(b + 10 * m);
+#pragma unroll
+		for(int k = 0; k < 5; ++k) {
+			const float2 va = __ldg(ga + k), vb = __ldg(gb + k);
+			C.G[j][2 * k] = pair(va.x, vb.x);
+			C.G[j][2 * k + 1] = pair(va.y, vb.y);
+		}
+		if constexpr(RT) {
+#pragma unroll
+			for(int k = 0; k < 4; ++k) {
+				const int f = extra_field(m, k, g.bug_gzz);
+				C.W[j][k] = f >= 0 ? pair(__ldg(a + f), __ldg(b + f)) : 0;
+			}
+		}
+	}
+}
+
+/* What a lane keeps of its axis (lanes 1-3) or of time (lane 0).  While x^m
+ * stays in [xa, xb) the cell held is the right one, so the RHS needs no
+ * search: w = (x - x0) inv + ci - ci.  The range is the cell cut to the box
+ * (lane 0: the times with the same levels in use), or empty. */
+struct Axis {
+	float x0, inv, ci; /* the cell's first node, 1/width and index       */
+	float xa, xb;
+	int tag;           /* the cell index (lane 0: level code) in Cell    */
+};
+
+/* the levels in use: bit 0 level 0, bit 1 level 1; a level of weight zero
+ * (t outside [t1, t2] in physics mode, where the factor is clamped) is not
+ * read */
+__device__ __forceinline__ int
+level_code(bool single, float ft)
+{
+	return single ? 1 : (ft < 1.0f ? 1 : 0) | (ft > 0.0f ? 2 : 0);
+}
+
+template <bool RT>
+__device__ __forceinline__ void
+forget(Axis &A, Cell<RT> &C)
+{
+	A.tag = -1;
+	A.xa = INFINITY; /* empty */
+#pragma unroll
+	for(int j = 0; j < 4; ++j) {
+#pragma unroll
+		for(int k = 0; k < 10; ++k)
+			C.G[j][k] = 0;
+		if constexpr(RT)
+#pragma unroll
+			for(int k = 0; k < 4; ++k)
+				C.W[j][k] = 0;
+	}
+}
+
+/* Contraction of both levels straight from memory, for a ray between the
+ * levels in a one-level launch (LV = 1): rare there by the launch rule. */
+template <bool RT>
+__device__ __noinline__ float2
+contract_both(const GridParams &g, int m, int ix, int iy, int iz, float4 w4, float4 u4)
+{
+	const float w[4] = {w4.x, w4.y, w4.z, w4.w}, u[4] = {u4.x, u4.y, u4.z, u4.w};
+	float G = 0.0f, K = 0.0f;
+#pragma unroll 1
+	for(int c = 0; c < 8; ++c) {
+		const float wc = ((c & 1) ? w[0] : 1.0f - w[0]) * ((c & 2) ? w[1] : 1.0f - w[1]) *
+		                 ((c & 4) ? w[2] : 1.0f - w[2]);
+		const int x = (c & 1) ? min(ix + 1, g.nx - 1) : ix;
+		const int y = (c & 2) ? min(iy + 1, g.ny - 1) : iy;
+		const int z = (c & 4) ? min(iz + 1, g.nz - 1) : iz;
+		const long long row = (((long long)z * g.ny + y) * g.nx + x) * GRAY_NSTRIDE;
+#pragma unroll 1
+		for(int l = 0; l < 2; ++l) {
+			const float wl = wc * (l ? w[3] : 1.0f - w[3]);
+			const float *src = g.lvl[l] + row;
+			const float2 *gs = (const float2 *)(src + 10 * m);
+			float s = 0.0f;
+			int k = 0;
+#pragma unroll
+			for(int i = 0; i < 4; ++i)
+#pragma unroll
+				for(int j = i; j < 4; ++j) {
+					const float uu = u[i] * u[j];
+					const float2 v = __ldg(gs + k / 2);
+					s = fmaf((k & 1) ? v.y : v.x, i == j ? uu : 2.0f * uu, s);
+					++k;
+				}
+			G = fmaf(wl, s, G);
+			if(RT) {
+				const float v1[4] = {1.0f, 0.0f, 0.0f, 0.0f};
+				const float *v = m == 1 ? v1 : u;
+				float e[4];
+#pragma unroll
+				for(int q = 0; q < 4; ++q) {
+					const int f = extra_field(m, q, g.bug_gzz);
+					e[q] = f >= 0 ? __ldg(src + f) : 0.0f;
+				}
+				const float kk = fmaf(e[3], v[3], fmaf(e[2], v[2], fmaf(e[1], v[1], e[0] * v[0])));
+				K = fmaf(wl, kk, K);
+			}
+		}
+	}
+	return make_float2(G, K);
+}
+
+/* The ray left its cell, entered or left the box, or changed levels:
+ * search, load what is missing, and set the range in which none of this is
+ * needed.  Returns w (lane 0: the time factor); in: inside the box. */
+template <int LV, bool RT>
+__device__ __forceinline__ float
+enter_cell(const GridParams &g, const DystConst &dc, Axis &A, Cell<RT> &C, int lane, bool on,
+           float xs, bool &in)
+{
+	constexpr int L = 4 * LV;
+	const unsigned FULL = 0xffffffffu;
+	const int m = lane & 3, l = (lane & (L - 1)) >> 2, first = lane & ~(L - 1);
+	const float lo = g.box[m], hi = g.box[m + 4];
+	in = true;
+	if(g.physics) {
+		const unsigned out = __ballot_sync(FULL, m > 0 && !(xs >= lo && xs <= hi));
+		in = ((out >> first) & ((1u << L) - 1u)) == 0;
+	}
+	const bool need = on && in;
+	float w = 0.0f;
+	int i0 = 0;
+	if(need) {
+		if(m == 0) {
+			if(!g.single) {
+				A.x0 = lo;
+				A.inv = rcp_a(hi - lo);
+				w = (xs - lo) * A.inv;
+				if(g.physics)
+					w = fminf(fmaxf(w, 0.0f), 1.0f);
+			}
+			i0 = level_code(g.single, w);
+			/* times at which the rounded factor surely gives the same code */
+			const float mg = 1e-5f * (fabsf(lo) + fabsf(hi));
+			A.xa = i0 == 2 ? hi + mg : i0 == 3 ? lo + mg : -INFINITY;
+			A.xb = i0 == 1 ? (g.single ? INFINITY : lo) : i0 == 3 ? hi - mg : INFINITY;
+			if(i0 == 0 || (LV == 1 && i0 == 3))
+				A.xa = INFINITY;
+		} else {
+			float uu;
+			if(xs >= A.xa && xs < A.xb) {
+				uu = fmaf(xs - A.x0, A.inv, A.ci);
+			} else {
+				const int n = m == 1 ? g.nx : m == 2 ? g.ny : g.nz;
+				float4 cell;
+				uu = axis_search(g.nodes_f[m - 1], n, xs, dc.B[m - 1], dc.iA[m - 1], cell);
+				A.x0 = cell.x;
+				A.inv = cell.z;
+				A.ci = cell.w;
+				A.xa = cell.x;
+				A.xb = cell.y;
+				if(g.physics) {
+					A.xa = fmaxf(A.xa, lo);
+					A.xb = fminf(A.xb, hi);
+				}
+			}
+			const float fl = floorf(uu);
+			i0 = (int)fl;
+			w = uu - fl;
+			if(fl != A.ci) /* rounded up to the next node: that cell, this once */
+				A.xa = INFINITY;
+		}
+	}
+	const unsigned moved = __ballot_sync(FULL, need && A.tag != i0);
+	if(moved) {
+		const int ix = __shfl_sync(FULL, i0, 1, 4), iy = __shfl_sync(FULL, i0, 2, 4),
+		          iz = __shfl_sync(FULL, i0, 3, 4), code = __shfl_sync(FULL, i0, 0, 4);
+		if((moved >> first) & ((1u << L) - 1u)) {
+			A.tag = i0;
+			if(LV == 1 ? code == 1 || code == 2 : (code >> l) & 1)
+				load_cell<RT>(g, g.lvl[LV == 1 ? code - 1 : l], m, ix, iy, iz, C);
+		}
+	}
+	return w;
+}
+
+/* Gamma^m_ab u^a u^b on lane m, and the acceleration du^m of dyst.cl:112-194
+ * from it.  All lanes of the warp take part; `on` marks the lanes whose ray
+ * steps.  Corners are summed in the order 000, 100, 010, ... with the levels
+ * of each corner in turn.  With RT also kn = {k_t, k_z, n_e}.  in: inside
+ * the box (or no box); all: so are all rays, in the cells they hold. */
+template <int LV, bool RT>
+__device__ __forceinline__ float
+dyst_accel(const GridParams &g, const DystConst &dc, Axis &A, Cell<RT> &C, int lane, bool on,
+           float xs, float us, float *kn, bool &in, bool &all)
+{
+	constexpr int L = 4 * LV;
+	const unsigned FULL = 0xffffffffu;
+	const int m = lane & 3, first = lane & ~(L - 1);
+	const float u0 = __shfl_sync(FULL, us, 0, 4), u1 = __shfl_sync(FULL, us, 1, 4),
+	            u2 = __shfl_sync(FULL, us, 2, 4), u3 = __shfl_sync(FULL, us, 3, 4);
+	float w = fmaf(xs - A.x0, A.inv, A.ci) - A.ci;
+	in = true;
+	all = __all_sync(FULL, !on || (xs >= A.xa && xs < A.xb && (w < 1.0f || (LV == 2 && m == 0))));
+	if(!all)
+		w = enter_cell<LV, RT>(g, dc, A, C, lane, on, xs, in);
+	else if(LV == 2 && m == 0 && g.physics)
+		w = fminf(fmaxf(w, 0.0f), 1.0f);
+	const bool need = on && in;
+	const float wx = __shfl_sync(FULL, w, 1, 4), wy = __shfl_sync(FULL, w, 2, 4),
+	            wz = __shfl_sync(FULL, w, 3, 4);
+
+	pair_t S2[4] = {0, 0, 0, 0};
+	{
+		const float u[4] = {u0, u1, u2, u3};
+		int k = 0;
+#pragma unroll
+		for(int i = 0; i < 4; ++i)
+#pragma unroll
+			for(int j = i; j < 4; ++j) {
+				const float uu = u[i] * u[j];
+				const float p = i == j ? uu : 2.0f * uu;
+				const pair_t p2 = pair(p, p);
+#pragma unroll
+				for(int q = 0; q < 4; ++q)
+					S2[q] = fma2(C.G[q][k], p2, S2[q]);
+				++k;
+			}
+	}
+	float2 S[4], K[4];
+#pragma unroll
+	for(int q = 0; q < 4; ++q)
+		S[q] = unpair(S2[q]);
+	if constexpr(RT) {
+		const bool rho = m == 1;
+		const float v0 = rho ? 1.0f : u0, v1 = rho ? 0.0f : u1, v2 = rho ? 0.0f : u2,
+		            v3 = rho ? 0.0f : u3;
+#pragma unroll
+		for(int q = 0; q < 4; ++q)
+			K[q] = unpair(fma2(C.W[q][3], pair(v3, v3),
+			              fma2(C.W[q][2], pair(v2, v2),
+			              fma2(C.W[q][1], pair(v1, v1), mul2(C.W[q][0], pair(v0, v0))))));
+	}
+	const float ax = 1.0f - wx, ay = 1.0f - wy, az = 1.0f - wz;
+	float G = 0.0f, Km = 0.0f;
+	if constexpr(LV == 1) {
+		/* one level in use: its time weight is exactly 1 (a single level, or
+		 * the clamped factor of physics mode) */
+#pragma unroll
+		for(int j = 0; j < 4; ++j) {
+			const float wy_ = (j & 1) ? wy : ay, wz_ = (j & 2) ? wz : az;
+			const float2 wc = unpair(mul2(mul2(pair(ax, wx), pair(wy_, wy_)), pair(wz_, wz_)));
+			G = fmaf(wc.x, S[j].x, G);
+			G = fmaf(wc.y, S[j].y, G);
+			if(RT) {
+				Km = fmaf(wc.x, K[j].x, Km);
+				Km = fmaf(wc.y, K[j].y, Km);
+			}
+		}
+		if(!all && !g.single) {
+			const int code = __shfl_sync(FULL, A.tag, 0, 4);
+			if(need && code != 1 && code != 2) {
+				G = Km = 0.0f;
+				if(code == 3) {
+					const unsigned gm = 0xfu << first;
+					const float ft = __shfl_sync(gm, w, 0, 4);
+					const float2 r = contract_both<RT>(g, m, __shfl_sync(gm, A.tag, 1, 4),
+					                                   __shfl_sync(gm, A.tag, 2, 4),
+					                                   __shfl_sync(gm, A.tag, 3, 4),
+					                                   make_float4(wx, wy, wz, ft),
+					                                   make_float4(u0, u1, u2, u3));
+					G = r.x;
+					Km = r.y;
+					forget(A, C); /* nothing of the cell is live across the call */
+				}
+			}
+		}
+	} else {
+		const float ft = __shfl_sync(FULL, w, 0, 4);
+		const int code = __shfl_sync(FULL, A.tag, 0, 4);
+		/* the other level's sums come from the ray's other four lanes; the
+		 * lanes of level 0 add both up */
+		const bool use0 = code & 1, use1 = code & 2;
+#pragma unroll
+		for(int c = 0; c < 8; ++c) {
+			const float wc = ((c & 1) ? wx : ax) * ((c & 2) ? wy : ay) * ((c & 4) ? wz : az);
+			const float s0 = (c & 1) ? S[c >> 1].y : S[c >> 1].x;
+			const float s1 = __shfl_xor_sync(FULL, s0, 4);
+			const float w0 = wc * (1.0f - ft), w1 = wc * ft;
+			G = use0 ? fmaf(w0, s0, G) : G;
+			G = use1 ? fmaf(w1, s1, G) : G;
+			if(RT) {
+				const float k0 = (c & 1) ? K[c >> 1].y : K[c >> 1].x;
+				const float k1 = __shfl_xor_sync(FULL, k0, 4);
+				Km = use0 ? fmaf(w0, k0, Km) : Km;
+				Km = use1 ? fmaf(w1, k1, Km) : Km;
+			}
+		}
+		G = __shfl_sync(FULL, G, m, L);
+	}
+	const float G0 = __shfl_sync(FULL, G, 0, L);
+	if constexpr(RT) {
+		kn[0] = __shfl_sync(FULL, Km, 0, L);
+		kn[1] = __shfl_sync(FULL, Km, 3, L);
+		kn[2] = __shfl_sync(FULL, Km, 1, L);
+		if(!in) { /* flat space, empty */
+			kn[0] = -u0;
+			kn[1] = u3;
+			kn[2] = 0.0f;
+		}
+	}
+	return fmaf(G0, us, -G);
+}
+
+/* Far from the box (physics mode): u is constant and a step is the
+ * compensated update of x alone, so a chunk of steps runs as one loop of
+ * four operations each: as many as every ray of the warp surely stays
+ * outside (by its distance to the box on some axis, less 1% for rounding
+ * and two steps for the stage positions) and short of its interval's last
+ * step.  k: the sum of the stages' slopes, dx: the size of one step.  False:
+ * no step was taken. */
+__device__ __forceinline__ bool
+flat_steps(const GridParams &g, int m, bool step, int &h, int n, int dh_step,
+           float h6, float k, float dx, float &xh, float &xl, float uh, float ul, unsigned &cnt)
+{
+	const unsigned FULL = 0xffffffffu;
+	/* steps until this lane's axis may reach the box; 0: it is inside */
+	const float lo = g.box[m], hi = g.box[m + 4];
+	const float d = m ? fmaxf(lo - xh, xh - hi) : 0.0f;
+	float far = d > 0.0f ? fminf(0.99f * d * rcp_a(dx + 1e-30f), 1e6f) - 2.0f : 0.0f;
+	far = fmaxf(far, __shfl_xor_sync(FULL, far, 1));
+	far = fmaxf(far, __shfl_xor_sync(FULL, far, 2));
+	/* u's own update must be a fixed point */
+	const float tu = uh - ul;
+	const bool still = tu == uh && (tu - uh) + ul == ul;
+	int todo = far >= 1.0f ? (int)far : 0;
+	const int left = step ? (n - h - 1) / dh_step : INT_MAX; /* not the last step */
+	todo = !step ? INT_MAX : still ? min(todo, left) : 0;
+	todo = __reduce_min_sync(FULL, todo);
+	if(todo <= 0 || todo == INT_MAX)
+		return false;
+	if(step) {
+		for(int i = 0; i < todo; ++i) {
+			const float yx = fmaf(h6, k, -xl);
+			const float tx = xh + yx;
+			xl = (tx - xh) - yx;
+			xh = tx;
+		}
+		h += todo * dh_step;
+		cnt += todo;
+	}
+	__syncwarp();
 	return true;
 }
 
-/* Gamma^mu_ab u^a u^b for mu = t,x,y,z from the 40 interpolated Gamma:
- * each corner's row is gathered with 32-byte loads and contracted with
- * u^a u^b before the trilinear weight is applied.
- * With RT, also the covariant momentum k_mu = g_mu,nu u^nu (dyst.cl:55-81,
- * with the g_zz flag of dyst.cl:78) and n_e = rho (flow.cl:48) into
- * kn[0..3] and kn[4], contracted per corner like Gamma. */
-template <bool RT = false>
-__device__ __forceinline__ void
-dyst_rhs32(const GridParams &g, const DystConst &dc, float4 *cells, const float *s, float *ds,
-           float *kn = nullptr)
+/* the null-constraint diagnostic of a finished ray, out of line so that its
+ * FP64 temporaries do not add to the registers of the stepping loop */
+__device__ __noinline__ double
+final_uu(const GridParams &g, double q0, double q1, double q2, double q3, double v0, double v1,
+         double v2, double v3)
 {
-	const float *u = s + 4;
-	ds[0] = u[0]; ds[1] = u[1]; ds[2] = u[2]; ds[3] = u[3];
-	if(g.physics && !inside32(g, s)) {
-		ds[4] = ds[5] = ds[6] = ds[7] = 0.0f;
-		if(RT) {
-			kn[0] = -u[0]; kn[1] = u[1]; kn[2] = u[2]; kn[3] = u[3];
-			kn[4] = 0.0f;
-		}
-		return;
-	}
-	int i0[3], i1[3];
-	float w[3];
-	const int n[3] = {g.nx, g.ny, g.nz};
-#pragma unroll
-	for(int a = 0; a < 3; ++a) {
-		float uu = axis_uvw32c(g, a, s[a + 1], dc.B[a], dc.iA[a], cells[a * CELL_STRIDE]);
-		float fl = floorf(uu);
-		i0[a] = (int)fl;
-		w[a] = uu - fl;
-		i1[a] = min(i0[a] + 1, n[a] - 1);
-	}
-	float ft = 0.0f;
-	if(!g.single) {
-		ft = (s[0] - g.box[0]) * rcp_a(g.box[4] - g.box[0]);
-		if(g.physics)
-			ft = fminf(fmaxf(ft, 0.0f), 1.0f);
-	}
-	/* u^a u^b over the 10 stored (a <= b) components, off-diagonal doubled */
-	float p[10];
-	{
-		int k = 0;
-#pragma unroll
-		for(int i = 0; i < 4; ++i)
-#pragma unroll
-			for(int j = i; j < 4; ++j) {
-				float uu = u[i] * u[j];
-				p[k++] = i == j ? uu : 2.0f * uu;
-			}
-	}
-	/* Interpolation and the contraction with u u are both linear, so each
-	 * corner's 40 Gamma are contracted first (4 sums) and only the sums are
-	 * weighted: 4 accumulators instead of 40 keeps registers for warps. */
-	float Gm[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-	float Km[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-	const float ax = 1.0f - w[0], ay = 1.0f - w[1], az = 1.0f - w[2];
-	/* a time level whose weight is zero (t outside [t1, t2] in physics
-	 * mode, where the factor is clamped) is not fetched at all */
-	const bool use0 = g.single || ft < 1.0f;
-	const bool use1 = !g.single && ft > 0.0f;
-#if GRAY_DYST_PREFETCH
-	if constexpr(!RT) {
-		/* the (corner, level) rows double-buffered in registers: the next
-		 * row's five loads are in flight while the current row is
-		 * contracted.  Built only with GRAY_DYST_PREFETCH=1: on
-		 * numerical_128 it measured 1.6x slower under the 128-register
-		 * cap (the second buffer spills) and 1.17x slower at 250 registers
-		 * (half the warps per SM) */
-		const int nl = (use0 ? 1 : 0) + (use1 ? 1 : 0), l0 = use0 ? 0 : 1, items = 8 * nl;
-		auto src_of = [&](int it) {
-			const int c = it / nl, l = l0 + it % nl;
-			const int ix = (c & 1) ? i1[0] : i0[0];
-			const int iy = (c & 2) ? i1[1] : i0[1];
-			const int iz = (c & 4) ? i1[2] : i0[2];
-			return g.lvl[l] + (((long long)iz * g.ny + iy) * g.nx + ix) * GRAY_NSTRIDE;
-		};
-		auto contract = [&](const F8 *v, int it) {
-			const int c = it / nl, l = l0 + it % nl;
-			float wl = ((c & 1) ? w[0] : ax) * ((c & 2) ? w[1] : ay) * ((c & 4) ? w[2] : az);
-			if(!g.single)
-				wl *= l ? ft : 1.0f - ft;
-			float sm[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-			for(int k = 0; k < 5; ++k)
-#pragma unroll
-				for(int q = 0; q < 8; ++q) {
-					const int idx = 8 * k + q;
-					sm[idx / 10] = fmaf(v[k].v[q], p[idx % 10], sm[idx / 10]);
-				}
-#pragma unroll
-			for(int m = 0; m < 4; ++m)
-				Gm[m] = fmaf(wl, sm[m], Gm[m]);
-		};
-		F8 A[5], B[5];
-		{
-			const float *s0 = src_of(0);
-#pragma unroll
-			for(int k = 0; k < 5; ++k)
-				A[k] = ldg8(s0 + 8 * k);
-		}
-#pragma unroll 1
-		for(int it = 0; it < items; it += 2) { /* items is 8 or 16 */
-			const float *sb = src_of(it + 1);
-#pragma unroll
-			for(int k = 0; k < 5; ++k)
-				B[k] = ldg8(sb + 8 * k);
-			contract(A, it);
-			if(it + 2 < items) {
-				const float *sa = src_of(it + 2);
-#pragma unroll
-				for(int k = 0; k < 5; ++k)
-					A[k] = ldg8(sa + 8 * k);
-			}
-			contract(B, it + 1);
-		}
-#pragma unroll
-		for(int m = 0; m < 4; ++m)
-			ds[4 + m] = fmaf(Gm[0], u[m], -Gm[m]);
-		return;
-	}
-#endif
-	/* one corner at a time: unrolling the eight corners buys no load
-	 * parallelism the 16 resident warps do not already give, and its
-	 * register pressure spills (measured 13% slower) */
-#pragma unroll 1
-	for(int c = 0; c < 8; ++c) {
-		float wc = ((c & 1) ? w[0] : ax) * ((c & 2) ? w[1] : ay) * ((c & 4) ? w[2] : az);
-		int ix = (c & 1) ? i1[0] : i0[0];
-		int iy = (c & 2) ? i1[1] : i0[1];
-		int iz = (c & 4) ? i1[2] : i0[2];
-		long long row = (((long long)iz * g.ny + iy) * g.nx + ix) * GRAY_NSTRIDE;
-		for(int l = 0; l < 2; ++l) {
-			if(!(l ? use1 : use0))
-				continue;
-			float wl = g.single ? wc : wc * (l ? ft : 1.0f - ft);
-			const float *src = g.lvl[l] + row;
-			float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-			for(int k = 0; k < 5; ++k) {
-				const F8 v = ldg8(src + 8 * k);
-#pragma unroll
-				for(int q = 0; q < 8; ++q) {
-					const int idx = 8 * k + q; /* Gamma^(idx/10)_(idx%10) */
-					s[idx / 10] = fmaf(v.v[q], p[idx % 10], s[idx / 10]);
-				}
-			}
-#pragma unroll
-			for(int m = 0; m < 4; ++m)
-				Gm[m] = fmaf(wl, s[m], Gm[m]);
-			if(RT) {
-				/* g_tt g_tx g_ty g_tz g_xx g_xy g_xz g_yy | g_yz g_zz rho pad */
-				const F8 ab = ldg8(src + 40), de = ldg8(src + 48);
-				const float4 a = make_float4(ab.v[0], ab.v[1], ab.v[2], ab.v[3]);
-				const float4 b = make_float4(ab.v[4], ab.v[5], ab.v[6], ab.v[7]);
-				const float4 d = make_float4(de.v[0], de.v[1], de.v[2], de.v[3]);
-				const float gzz = g.bug_gzz ? d.x : d.y;
-				const float k0 = fmaf(a.w, u[3], fmaf(a.z, u[2], fmaf(a.y, u[1], a.x * u[0])));
-				const float k1 = fmaf(b.z, u[3], fmaf(b.y, u[2], fmaf(b.x, u[1], a.y * u[0])));
-				const float k2 = fmaf(d.x, u[3], fmaf(b.w, u[2], fmaf(b.y, u[1], a.z * u[0])));
-				const float k3 = fmaf(gzz, u[3], fmaf(d.x, u[2], fmaf(b.z, u[1], a.w * u[0])));
-				Km[0] = fmaf(wl, k0, Km[0]);
-				Km[1] = fmaf(wl, k1, Km[1]);
-				Km[2] = fmaf(wl, k2, Km[2]);
-				Km[3] = fmaf(wl, k3, Km[3]);
-				Km[4] = fmaf(wl, d.z, Km[4]);
-			}
-		}
-	}
-#pragma unroll
-	for(int m = 0; m < 4; ++m)
-		ds[4 + m] = fmaf(Gm[0], u[m], -Gm[m]);
-	if(RT) {
-#pragma unroll
-		for(int m = 0; m < 5; ++m)
-			kn[m] = Km[m];
-	}
+	const double s[8] = {q0, q1, q2, q3, v0, v1, v2, v3};
+	return dyst_getuu64(g, s);
 }
 
-/* ------------------------------------------ gathers staged in shared memory */
+constexpr int DYST_BLOCK = 128;
 
-/* The same geodesic RHS with the corner rows staged through shared memory:
- * each (corner, level) row of 40 Gamma is copied global -> shared with ten
- * 16-byte cp.async (through L1, .ca) into a per-thread double buffer, and
- * the copy of the next row is in flight while the current one is
- * contracted.  The loads then hold no registers while they wait, so more of
- * them overlap than the register-resident form allows at 16 warps per SM.
- * Buffer layout [stage][chunk][thread] of float4: a warp's LDS.128 of one
- * chunk touches 32 consecutive float4, without bank conflicts.
- *
- * Built only with GRAY_DYST_STAGED=1: on numerical_128 it measured 5.2x
- * slower than the register gathers.  Its 80 KiB of shared memory per block
- * come out of the same on-chip storage as L1, and the rows that hit L1 95%
- * of the time in the register form then come from L2. */
-constexpr int STAGE_CHUNKS = 10; /* 40 floats = 10 x 16 bytes */
-
-__device__ __forceinline__ void
-cp_async16(float4 *dst, const float *src)
+/* LV: the time levels a ray's lanes hold; FPL: frequencies
+ * per lane (0: geodesics alone).  The transfer pairs (I, tau) are FP64 and
+ * ride along in the same RK4 stages. */
+template <int LV, int FPL>
+__global__ void __launch_bounds__(DYST_BLOCK, 3)
+dyst_mixed_kernel(const MixedTable T, const __grid_constant__ GridParams g, const DystConst dc,
+                  const int nf, unsigned int *__restrict__ queue,
+                  unsigned long long *__restrict__ steps, unsigned long long *__restrict__ inbox)
 {
-	const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-	asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-}
-
-__device__ __forceinline__ void
-cp_async_commit()
-{
-	asm volatile("cp.async.commit_group;" ::: "memory");
-}
-
-template <int N>
-__device__ __forceinline__ void
-cp_async_wait()
-{
-	asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-__device__ __forceinline__ void
-dyst_rhs32_staged(const GridParams &g, const DystConst &dc, float4 *cells, float4 *stage,
-                  const float *s, float *ds)
-{
-	const float *u = s + 4;
-	ds[0] = u[0]; ds[1] = u[1]; ds[2] = u[2]; ds[3] = u[3];
-	if(g.physics && !inside32(g, s)) {
-		ds[4] = ds[5] = ds[6] = ds[7] = 0.0f;
-		return;
-	}
-	int i0[3], i1[3];
-	float w[3];
-	const int n[3] = {g.nx, g.ny, g.nz};
-#pragma unroll
-	for(int a = 0; a < 3; ++a) {
-		float uu = axis_uvw32c(g, a, s[a + 1], dc.B[a], dc.iA[a], cells[a * CELL_STRIDE]);
-		float fl = floorf(uu);
-		i0[a] = (int)fl;
-		w[a] = uu - fl;
-		i1[a] = min(i0[a] + 1, n[a] - 1);
-	}
-	float ft = 0.0f;
-	if(!g.single) {
-		ft = (s[0] - g.box[0]) * rcp_a(g.box[4] - g.box[0]);
-		if(g.physics)
-			ft = fminf(fmaxf(ft, 0.0f), 1.0f);
-	}
-	float p[10];
-	{
-		int k = 0;
-#pragma unroll
-		for(int i = 0; i < 4; ++i)
-#pragma unroll
-			for(int j = i; j < 4; ++j) {
-				float uu = u[i] * u[j];
-				p[k++] = i == j ? uu : 2.0f * uu;
-			}
-	}
-	float Gm[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-	const float ax = 1.0f - w[0], ay = 1.0f - w[1], az = 1.0f - w[2];
-	const bool use0 = g.single || ft < 1.0f;
-	const bool use1 = !g.single && ft > 0.0f;
-	/* the (corner, level) rows to gather: corner-major, levels in order */
-	const int nl = (use0 ? 1 : 0) + (use1 ? 1 : 0);
-	const int l0 = use0 ? 0 : 1;
-	const int items = 8 * nl;
-	auto row_of = [&](int it) {
-		const int c = it / nl, l = l0 + it % nl;
-		const int ix = (c & 1) ? i1[0] : i0[0];
-		const int iy = (c & 2) ? i1[1] : i0[1];
-		const int iz = (c & 4) ? i1[2] : i0[2];
-		return g.lvl[l] + (((long long)iz * g.ny + iy) * g.nx + ix) * GRAY_NSTRIDE;
-	};
-	auto issue = [&](int it) {
-		const float *src = row_of(it);
-		float4 *dst = stage + (it & 1) * STAGE_CHUNKS * CELL_STRIDE;
-#pragma unroll
-		for(int k = 0; k < STAGE_CHUNKS; ++k)
-			cp_async16(dst + k * CELL_STRIDE, src + 4 * k);
-		cp_async_commit();
-	};
-	issue(0);
-#pragma unroll 1
-	for(int it = 0; it < items; ++it) {
-		if(it + 1 < items) {
-			issue(it + 1);
-			cp_async_wait<1>(); /* row it has landed, row it + 1 in flight */
-		} else {
-			cp_async_wait<0>();
-		}
-		const int c = it / nl, l = l0 + it % nl;
-		float wl = ((c & 1) ? w[0] : ax) * ((c & 2) ? w[1] : ay) * ((c & 4) ? w[2] : az);
-		if(!g.single)
-			wl *= l ? ft : 1.0f - ft;
-		const float4 *src = stage + (it & 1) * STAGE_CHUNKS * CELL_STRIDE;
-		float sm[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-		for(int k = 0; k < STAGE_CHUNKS; ++k) {
-			const float4 v = src[k * CELL_STRIDE];
-			const float vv[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-			for(int q = 0; q < 4; ++q) {
-				const int idx = 4 * k + q; /* Gamma^(idx/10)_(idx%10) */
-				sm[idx / 10] = fmaf(vv[q], p[idx % 10], sm[idx / 10]);
-			}
-		}
-#pragma unroll
-		for(int m = 0; m < 4; ++m)
-			Gm[m] = fmaf(wl, sm[m], Gm[m]);
-	}
-#pragma unroll
-	for(int m = 0; m < 4; ++m)
-		ds[4 + m] = fmaf(Gm[0], u[m], -Gm[m]);
-}
-
-/* NF > 0: the thermal transfer pairs (I, tau) ride along in FP64 (rt[],
- * first the NF intensities, then the NF optical depths), integrated by the
- * same RK4 stages with the FP64 emissivities of thermal.cuh on the FP32
- * momentum and density; the stages run as a rolled loop so that the FP64
- * transfer is instantiated once. */
-template <int NF, bool STAGED>
-__global__ void __launch_bounds__(256, NF == 0 ? 2 : 1)
-dyst_mixed_kernel(const MixedTable T, const GridParams g, const DystConst dc,
-                  unsigned int *__restrict__ queue, unsigned long long *__restrict__ steps,
-                  unsigned long long *__restrict__ inbox)
-{
-	static_assert(!STAGED || NF == 0, "staged gathers: geodesic-only renders");
-	extern __shared__ float4 s_stage[]; /* STAGED: 2 x STAGE_CHUNKS x CELL_STRIDE */
-	float4 *stage = s_stage + threadIdx.x;
-	constexpr int ND = 8;            /* FP32 geodesic state           */
-	constexpr int NR = 2 * NF;       /* FP64 transfer state           */
+	constexpr int L = 4 * LV;   /* lanes per ray */
+	constexpr bool RT = FPL > 0;
+	/* stages unrolled: 197 ms against 225 on the 512^2 render; with the
+	 * transfer one body measures faster (17.5 ms against 20.4) */
+	constexpr int STAGES = RT ? 1 : 4;
+	constexpr int NR = RT ? FPL : 1;
 	const unsigned FULL = 0xffffffffu;
-	const int lane = threadIdx.x & 31;
-	/* each thread's last cell per axis (axis_uvw32c); empty to start */
-	__shared__ float4 s_cells[3 * CELL_STRIDE];
-	float4 *cells = s_cells + threadIdx.x;
+	const int lane = threadIdx.x & 31, sub = lane & (L - 1), m = lane & 3;
+	const int first = lane & ~(L - 1);
+	const unsigned gmask = ((L == 32 ? 0u : (1u << L)) - 1u) << first;
+
+	Axis A;
+	Cell<RT> C;
+	forget(A, C);
+	A.x0 = A.inv = A.ci = A.xb = 0.0f;
+
+	float xh = 0.0f, xl = 0.0f, uh = 0.0f, ul = 0.0f; /* x^m, u^m: high and low parts */
+	double I[NR], tau[NR], nu[NR];
 #pragma unroll
-	for(int a = 0; a < 3; ++a)
-		cells[a * CELL_STRIDE] = make_float4(INFINITY, -INFINITY, 0.0f, 0.0f);
-	float hi[ND], lo[ND];
-	double rt[NR > 0 ? NR : 1];
-	long long ray = 0;
+	for(int i = 0; i < NR; ++i)
+		I[i] = tau[i] = nu[i] = 0.0;
+	unsigned ray = 0;
 	int dump = 0, h = 0, dh_step = 0, n = 0;
 	float dtn = 0.0f;
 	double dtnd = 0.0; /* the FP64 substep unit of the transfer */
-	bool active = false, exhausted = false;
-	unsigned long long cnt = 0, cnt_in = 0; /* all steps; steps that interpolate */
+	bool active = false, exhausted = false, bad = false;
+	bool quiet = false; /* every ray of the warp stayed in its cell and the box */
+	/* steps of the rays this lane leads, flushed at dump boundaries once a
+	 * count reaches 2^31: an interval takes fewer than 2^31 steps */
+	unsigned cnt = 0, cnt_in = 0;
 	const MixedRender *c = nullptr;
 
 	for(;;) {
-		bool need = !active && !exhausted;
-		unsigned mask = __ballot_sync(FULL, need);
-		if(mask) {
-			int leader = __ffs(mask) - 1;
-			unsigned base = 0;
-			if(lane == leader)
-				base = atomicAdd(queue, (unsigned)__popc(mask));
-			base = __shfl_sync(FULL, base, leader);
-			if(need) {
-				unsigned long long gidx = (unsigned long long)base +
-				                          __popc(mask & ((1u << lane) - 1));
-				if(gidx < T.total) {
-					int rr = 0;
-					while(rr + 1 < T.n_renders && T.prefix[rr + 1] <= gidx)
-						++rr;
-					c = &T.renders[rr];
-					ray = (long long)(gidx - T.prefix[rr]);
-					n = (int)((INT_MAX / c->n_sub) * c->n_sub);
+		if(!__all_sync(FULL, active)) {
+			const bool need = !active && !exhausted;
+			const unsigned mask = __ballot_sync(FULL, need && sub == 0);
+			if(mask) {
+				const int leader = __ffs(mask) - 1;
+				unsigned base = 0;
+				if(lane == leader)
+					base = atomicAdd(queue, (unsigned)__popc(mask));
+				base = __shfl_sync(FULL, base, leader);
+				if(need) {
+					const unsigned long long gidx = (unsigned long long)base +
+					                                __popc(mask & ((1u << first) - 1u));
+					if(gidx < T.total) {
+						int rr = 0;
+						while(rr + 1 < T.n_renders && T.prefix[rr + 1] <= gidx)
+							++rr;
+						c = &T.renders[rr];
+						ray = (unsigned)(gidx - T.prefix[rr]);
+						n = (int)((INT_MAX / c->n_sub) * c->n_sub);
+						const double vx = c->data[m * c->n_rays + ray];
+						const double vu = c->data[(4 + m) * c->n_rays + ray];
+						xh = (float)vx;
+						xl = (float)((double)xh - vx);
+						uh = (float)vu;
+						ul = (float)((double)uh - vu);
+						if constexpr(RT) {
 #pragma unroll
-					for(int k = 0; k < ND; ++k) {
-						double v = c->data[k * c->n_rays + ray];
-						hi[k] = (float)v;
-						lo[k] = (float)((double)hi[k] - v);
+							for(int i = 0; i < FPL; ++i) {
+								const int f = sub + i * L < nf ? sub + i * L : 0;
+								I[i] = c->data[(8 + f) * c->n_rays + ray];
+								tau[i] = c->data[(8 + nf + f) * c->n_rays + ray];
+								nu[i] = c->nu_hz[f];
+							}
+						}
+						dump = c->dump_begin - 1;
+						h = n; /* forces the first dump set-up below */
+						active = true;
+					} else {
+						exhausted = true;
 					}
-#pragma unroll
-					for(int k = 0; k < NR; ++k)
-						rt[k] = c->data[(ND + k) * c->n_rays + ray];
-					dump = c->dump_begin - 1;
-					h = n; /* forces the first dump set-up below */
-					active = true;
-				} else {
-					exhausted = true;
 				}
+				__syncwarp();
+			}
+			if(!__any_sync(FULL, active))
+				break;
+		}
+		bool step = active;
+		if(active && h >= n) { /* next dump interval: constants of driver.cl:93 */
+			step = false;
+			if(cnt >= 0x80000000u) {
+				if(sub == 0)
+					atomicAdd(steps, (unsigned long long)cnt);
+				cnt = 0;
+			}
+			if(cnt_in >= 0x80000000u) {
+				if(sub == 0 && inbox)
+					atomicAdd(inbox, (unsigned long long)cnt_in);
+				cnt_in = 0;
+			}
+			if(bad || ++dump >= c->dump_end) { /* done: write the ray back */
+				const double x = (double)xh - (double)xl, u = (double)uh - (double)ul;
+				double q[4], v[4];
+#pragma unroll
+				for(int k = 0; k < 4; ++k) {
+					q[k] = __shfl_sync(gmask, x, k, 4);
+					v[k] = __shfl_sync(gmask, u, k, 4);
+				}
+				if(sub < 4) {
+					c->data[m * c->n_rays + ray] = x;
+					c->data[(4 + m) * c->n_rays + ray] = u;
+				}
+				if constexpr(RT) {
+#pragma unroll
+					for(int i = 0; i < FPL; ++i)
+						if(sub + i * L < nf) {
+							c->data[(8 + sub + i * L) * c->n_rays + ray] = I[i];
+							c->data[(8 + nf + sub + i * L) * c->n_rays + ray] = tau[i];
+						}
+				}
+				if(sub == 0)
+					c->info[ray] = bad ? q[0] - q[0] /* NaN marks the ray */
+					                   : final_uu(g, q[0], q[1], q[2], q[3], v[0], v[1], v[2], v[3]);
+				active = bad = false;
+				forget(A, C); /* nothing of the cell is live across the call */
+			} else {
+				double t0 = c->t_init + (double)dump * c->dt_dump;
+				double t1 = c->t_init + (double)(dump + 1) * c->dt_dump;
+				double dt = t1 - t0;
+				dh_step = (int)(dyst_getdt64(dt / (double)c->n_sub) / dt * (double)n);
+				dtnd = dt / (double)n;
+				dtn = (float)dtnd;
+				h = 0;
+				if(dh_step <= 0) /* zero-length interval: nothing to integrate */
+					h = n;
+				else
+					step = true;
 			}
 		}
-		if(!__any_sync(FULL, active))
-			break;
-		if(!active)
-			continue;
-		if(h >= n) { /* next dump interval: constants of driver.cl:93 */
-			if(++dump >= c->dump_end) {
-				double s[ND];
-#pragma unroll
-				for(int k = 0; k < ND; ++k) {
-					s[k] = (double)hi[k] - (double)lo[k];
-					c->data[k * c->n_rays + ray] = s[k];
-				}
-#pragma unroll
-				for(int k = 0; k < NR; ++k)
-					c->data[(ND + k) * c->n_rays + ray] = rt[k];
-				c->info[ray] = dyst_getuu64(g, s);
-				active = false;
-				continue;
-			}
-			double t0 = c->t_init + (double)dump * c->dt_dump;
-			double t1 = c->t_init + (double)(dump + 1) * c->dt_dump;
-			double dt = t1 - t0;
-			dh_step = (int)(dyst_getdt64(dt / (double)c->n_sub) / dt * (double)n);
-			dtnd = dt / (double)n;
-			dtn = (float)dtnd;
-			h = 0;
-			if(dh_step <= 0) { /* zero-length interval: nothing to integrate */
-				h = n;
-				continue;
-			}
-		}
-		int dh = dh_step < n - h ? dh_step : n - h;
+		__syncwarp();
+		const int dh = step ? (dh_step < n - h ? dh_step : n - h) : 0;
 		const float hs = (float)dh * dtn, hh = 0.5f * hs;
-		float k[ND], t[ND], sum[ND];
-		cnt_in += (!g.physics || inside32(g, hi)) ? 1 : 0;
-		if constexpr(NF > 0) {
-			const double hsd = (double)dh * dtnd;
-			double trt[NR], srt[NR], krt[NR];
-#pragma unroll
-			for(int i = 0; i < ND; ++i)
-				t[i] = hi[i];
-#pragma unroll
-			for(int i = 0; i < NR; ++i)
-				trt[i] = rt[i];
-#pragma unroll 1
-			for(int st = 0; st < 4; ++st) {
-				float kn[5];
-				dyst_rhs32<true>(g, dc, cells, t, k, kn);
-				const double kd[4] = {kn[0], kn[1], kn[2], kn[3]};
-				rt_rhs_fast<NF>(c->tf, c->nu_hz, kd, (double)kn[4], trt + NF, krt, krt + NF);
-				const float wg = (st == 1 || st == 2) ? 2.0f : 1.0f;
-				const float cg = st < 2 ? hh : hs;
-				const double wd = wg, cd = st < 2 ? 0.5 * hsd : hsd;
-#pragma unroll
-				for(int i = 0; i < ND; ++i) { /* k4 stays in k for the update */
-					if(st < 3)
-						sum[i] = st == 0 ? k[i] : fmaf(wg, k[i], sum[i]);
-					t[i] = fmaf(cg, k[i], hi[i]);
-				}
-#pragma unroll
-				for(int i = 0; i < NR; ++i) {
-					srt[i] = st == 0 ? krt[i] : fma(wd, krt[i], srt[i]);
-					trt[i] = fma(cd, krt[i], rt[i]);
-				}
-			}
-#pragma unroll
-			for(int i = 0; i < NR; ++i)
-				rt[i] = fma(hsd / 6.0, srt[i], rt[i]);
-		} else {
-		auto geo = [&](const float *sv, float *kv) {
-			if constexpr(STAGED)
-				dyst_rhs32_staged(g, dc, cells, stage, sv, kv);
-			else
-				dyst_rhs32(g, dc, cells, sv, kv);
-		};
-		geo(hi, k);
-#pragma unroll
-		for(int i = 0; i < ND; ++i) {
-			sum[i] = k[i];
-			t[i] = fmaf(hh, k[i], hi[i]);
-		}
-		geo(t, k);
-#pragma unroll
-		for(int i = 0; i < ND; ++i) {
-			sum[i] = fmaf(2.0f, k[i], sum[i]);
-			t[i] = fmaf(hh, k[i], hi[i]);
-		}
-		geo(t, k);
-#pragma unroll
-		for(int i = 0; i < ND; ++i) {
-			sum[i] = fmaf(2.0f, k[i], sum[i]);
-			t[i] = fmaf(hs, k[i], hi[i]);
-		}
-		geo(t, k);
-		}
 		const float h6 = hs * (1.0f / 6.0f);
-		bool bad = false;
-#pragma unroll
-		for(int i = 0; i < ND; ++i) {
-			float inc = h6 * (sum[i] + k[i]);
-			float yv = inc - lo[i];
-			float tv = hi[i] + yv;
-			lo[i] = (tv - hi[i]) - yv;
-			hi[i] = tv;
-			bad |= !(fabsf(tv) <= FLT_MAX);
+
+		/* flat space through the whole step (physics mode outside the box):
+		 * no field enters, u is constant.  Not asked where the last step
+		 * found every ray inside. */
+		bool out = false, in0 = true, in = true; /* out: this ray, all step long */
+		bool flat = false;
+		if(!RT && g.physics && !quiet) {
+			const float lo = g.box[m], hi = g.box[m + 4];
+			auto outside = [&](float x) {
+				unsigned b = __ballot_sync(FULL, m > 0 && !(x >= lo && x <= hi));
+				return ((b >> first) & ((1u << L) - 1u)) != 0;
+			};
+			const bool o1 = outside(xh), o2 = outside(fmaf(hh, uh, xh)), o4 = outside(fmaf(hs, uh, xh));
+			out = o1 && o2 && o4;
+			flat = __all_sync(FULL, !step || out);
 		}
-		++cnt;
-		h += dh;
-		if(bad) { /* NaN/Inf (inside the singular region): ray done */
-			double s[ND];
+		float sx, su, kx, ku;
+		if(flat) {
+			sx = fmaf(2.0f, uh, fmaf(2.0f, uh, uh));
+			kx = uh;
+			su = ku = 0.0f;
+			in0 = false;
+			if(flat_steps(g, m, step, h, n, dh_step, h6, sx + kx, fabsf(hs * uh), xh, xl, uh, ul,
+			              cnt))
+				continue;
+		} else {
+			float kn[3];
+			bool all = true;
+			quiet = true;
+			double Is[NR], ts[NR], dI[NR], dtau[NR], st[NR];
+			const double hsd = (double)dh * dtnd;
+			sx = su = 0.0f;
+			float x = xh, u = uh;
 #pragma unroll
-			for(int kk = 0; kk < ND; ++kk) {
-				s[kk] = (double)hi[kk] - (double)lo[kk];
-				c->data[kk * c->n_rays + ray] = s[kk];
+			for(int i = 0; i < NR; ++i) {
+				st[i] = tau[i];
+				Is[i] = ts[i] = 0.0;
 			}
+#pragma unroll STAGES
+			for(int s = 0; s < 4; ++s) {
+				kx = u;
+				ku = dyst_accel<LV, RT>(g, dc, A, C, lane, step && !out, x, u, kn, in, all);
+				in = in && !out;
+				quiet = quiet && all;
+				in0 = s == 0 ? in : in0;
+				ku = in ? ku : 0.0f;
+				const float wg = (s == 1 || s == 2) ? 2.0f : 1.0f;
+				const float cg = s < 2 ? hh : hs;
+				if constexpr(RT) {
+					const double wd = wg, cd = s < 2 ? 0.5 * hsd : hsd;
+					if(step)
+						rt_rhs_fast<NR>(c->tf, nu, (double)kn[0], (double)kn[1],
+						                (double)kn[2], st, dI, dtau);
 #pragma unroll
-			for(int kk = 0; kk < NR; ++kk)
-				c->data[(ND + kk) * c->n_rays + ray] = rt[kk];
-			c->info[ray] = s[0] - s[0]; /* NaN marks the ray */
-			active = false;
+					for(int i = 0; i < NR; ++i) {
+						Is[i] = s == 0 ? dI[i] : fma(wd, dI[i], Is[i]);
+						ts[i] = s == 0 ? dtau[i] : fma(wd, dtau[i], ts[i]);
+						st[i] = fma(cd, dtau[i], tau[i]);
+					}
+				}
+				if(s < 3) { /* k4 stays in kx, ku for the update */
+					sx = s == 0 ? kx : fmaf(wg, kx, sx);
+					su = s == 0 ? ku : fmaf(wg, ku, su);
+				}
+				x = fmaf(cg, kx, xh);
+				u = fmaf(cg, ku, uh);
+			}
+			quiet = quiet && __all_sync(FULL, !out);
+			if constexpr(RT) {
+				if(step) {
+#pragma unroll
+					for(int i = 0; i < NR; ++i) {
+						I[i] = fma(hsd / 6.0, Is[i], I[i]);
+						tau[i] = fma(hsd / 6.0, ts[i], tau[i]);
+					}
+				}
+			}
 		}
+		/* compensated update, value = hi - lo */
+		const float yx = fmaf(h6, sx + kx, -xl), yu = fmaf(h6, su + ku, -ul);
+		const float tx = xh + yx, tu = uh + yu;
+		const bool badl = !(fabsf(tx) <= FLT_MAX) || !(fabsf(tu) <= FLT_MAX);
+		if(step) {
+			xl = (tx - xh) - yx;
+			xh = tx;
+			ul = (tu - uh) - yu;
+			uh = tu;
+			++cnt;
+			cnt_in += in0 ? 1 : 0;
+			h += dh;
+		}
+		const unsigned badm = __ballot_sync(FULL, step && badl);
+		if(badm & gmask) { /* NaN/Inf (inside the singular region): ray done */
+			bad = true;
+			h = n;
+		}
+		__syncwarp();
 	}
+	unsigned long long total = sub == 0 ? cnt : 0, total_in = sub == 0 ? cnt_in : 0;
 #pragma unroll
 	for(int o = 16; o > 0; o >>= 1) {
-		cnt += __shfl_xor_sync(FULL, cnt, o);
-		cnt_in += __shfl_xor_sync(FULL, cnt_in, o);
+		total += __shfl_xor_sync(FULL, total, o);
+		total_in += __shfl_xor_sync(FULL, total_in, o);
 	}
-	if(lane == 0 && cnt)
-		atomicAdd(steps, cnt);
-	if(lane == 0 && cnt_in && inbox)
-		atomicAdd(inbox, cnt_in);
+	if(lane == 0 && total)
+		atomicAdd(steps, total);
+	if(lane == 0 && total_in && inbox)
+		atomicAdd(inbox, total_in);
 }
 
-template <int NF, bool STAGED>
+template <int LV, int FPL>
 cudaError_t
-launch_dyst_nfs(const MixedTable &T, const GridParams &g, const DystConst &dc,
-                unsigned int *queue, unsigned long long *steps, cudaStream_t st,
-                const MixedLaunch &cfg, unsigned long long *inbox)
+launch_dyst(const MixedTable &T, const GridParams &g, const DystConst &dc, int nf,
+            unsigned int *queue, unsigned long long *steps, cudaStream_t st,
+            const MixedLaunch &cfg, unsigned long long *inbox)
 {
-	int block = cfg.block > 0 ? cfg.block : 256;
-	if(block > 256)
-		return cudaErrorInvalidValue; /* __launch_bounds__(256) */
-	/* the stage is indexed with the CELL_STRIDE of the launch bound */
-	const size_t smem = STAGED ? 2 * STAGE_CHUNKS * CELL_STRIDE * sizeof(float4) : 0;
-	cudaError_t e = cudaSuccess;
-	if(STAGED)
-		e = cudaFuncSetAttribute(dyst_mixed_kernel<NF, STAGED>,
-		                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+	const int sms = cfg.sms > 0 ? cfg.sms : 148;
+	const int max_block = cfg.block > 0 && cfg.block < DYST_BLOCK ? cfg.block : DYST_BLOCK;
+	/* few rays: one warp per block until every SM has a warp, so that a
+	 * small render's warps do not share an SM while others idle */
+	const unsigned long long warps = (T.total + 32 / (4 * LV) - 1) / (32 / (4 * LV));
+	int block = max_block;
+	if(warps < (unsigned long long)sms * (max_block / 32))
+		block = 32 * (int)((warps + sms - 1) / sms);
+	int occ = 0;
+	cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+		&occ, dyst_mixed_kernel<LV, FPL>, block, 0);
 	if(e != cudaSuccess)
 		return e;
 	int per_sm = cfg.blocks_per_sm;
-	if(per_sm <= 0) {
-		e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dyst_mixed_kernel<NF, STAGED>,
-		                                                  block, smem);
-		if(e != cudaSuccess)
-			return e;
-		if(per_sm <= 0)
-			per_sm = 1;
-	}
-	long long want = (long long)per_sm * (cfg.sms > 0 ? cfg.sms : 148);
-	long long need = (long long)((T.total + block - 1) / block);
+	if(per_sm <= 0 || per_sm > occ)
+		per_sm = occ > 0 ? occ : 1;
+	const long long want = (long long)per_sm * sms;
+	const long long need = (long long)((warps + block / 32 - 1) / (block / 32));
 	unsigned grid = (unsigned)(want < need ? want : need);
 	if(grid == 0)
 		grid = 1;
-	dyst_mixed_kernel<NF, STAGED><<<grid, block, smem, st>>>(T, g, dc, queue, steps, inbox);
+	dyst_mixed_kernel<LV, FPL><<<grid, block, 0, st>>>(T, g, dc, nf, queue, steps, inbox);
 	return cudaGetLastError();
-}
-
-#ifndef GRAY_DYST_STAGED
-#define GRAY_DYST_STAGED 0
-#endif
-
-template <int NF>
-cudaError_t
-launch_dyst_nf(const MixedTable &T, const GridParams &g, const DystConst &dc,
-               unsigned int *queue, unsigned long long *steps, cudaStream_t st,
-               const MixedLaunch &cfg, unsigned long long *inbox)
-{
-	if constexpr(NF == 0)
-		if(GRAY_DYST_STAGED)
-			return launch_dyst_nfs<0, true>(T, g, dc, queue, steps, st, cfg, inbox);
-	return launch_dyst_nfs<NF, false>(T, g, dc, queue, steps, st, cfg, inbox);
 }
 
 } /* namespace */
 
+/* Whether any ray of the renders may run between the two time levels, where
+ * both have weight: always in reference semantics (time extrapolates), and
+ * in physics mode if an affine window overlaps the levels' times (a ray's
+ * time is its affine parameter counted from the camera, dyst.cl:106). */
+bool
+dyst_between(const GridParams &g, const MixedRender *r, int n)
+{
+	if(g.single)
+		return false;
+	if(!g.physics)
+		return true;
+	for(int i = 0; i < n; ++i) {
+		const double a = r[i].t_init + (double)r[i].dump_begin * r[i].dt_dump;
+		const double b = r[i].t_init + (double)r[i].dump_end * r[i].dt_dump;
+		if((a < b ? a : b) < (double)g.box[4] && (a < b ? b : a) > (double)g.box[0])
+			return true;
+	}
+	return false;
+}
+
 cudaError_t
 launch_dyst_mixed_table(const MixedTable &T, const GridParams &g, int n_freq,
                         unsigned int *queue, unsigned long long *steps, cudaStream_t st,
-                        const MixedLaunch &cfg, unsigned long long *inbox)
+                        const MixedLaunch &cfg, bool between, unsigned long long *inbox)
 {
-	static_assert(GRAY_MAX_FREQ == 8, "one instantiation per frequency count");
+	static_assert(GRAY_MAX_FREQ == 8, "two frequencies per lane at most");
 	DystConst dc;
 	for(int a = 0; a < 3; ++a) {
 		dc.B[a] = (float)g.B[a];
@@ -812,19 +967,15 @@ launch_dyst_mixed_table(const MixedTable &T, const GridParams &g, int n_freq,
 	}
 	if(n_freq < 0 || n_freq > GRAY_MAX_FREQ)
 		return cudaErrorInvalidValue;
+	if(cfg.block > 256)
+		return cudaErrorInvalidValue;
 	cudaError_t e = cudaMemsetAsync(queue, 0, sizeof(unsigned int), st);
 	if(e != cudaSuccess)
 		return e;
-	switch(n_freq) {
-	case 0: return launch_dyst_nf<0>(T, g, dc, queue, steps, st, cfg, inbox);
-	case 1: return launch_dyst_nf<1>(T, g, dc, queue, steps, st, cfg, inbox);
-	case 2: return launch_dyst_nf<2>(T, g, dc, queue, steps, st, cfg, inbox);
-	case 3: return launch_dyst_nf<3>(T, g, dc, queue, steps, st, cfg, inbox);
-	case 4: return launch_dyst_nf<4>(T, g, dc, queue, steps, st, cfg, inbox);
-	case 5: return launch_dyst_nf<5>(T, g, dc, queue, steps, st, cfg, inbox);
-	case 6: return launch_dyst_nf<6>(T, g, dc, queue, steps, st, cfg, inbox);
-	case 7: return launch_dyst_nf<7>(T, g, dc, queue, steps, st, cfg, inbox);
-	default: return launch_dyst_nf<8>(T, g, dc, queue, steps, st, cfg, inbox);
-	}
+	if(between)
+		return n_freq == 0 ? launch_dyst<2, 0>(T, g, dc, n_freq, queue, steps, st, cfg, inbox)
+		                   : launch_dyst<2, 1>(T, g, dc, n_freq, queue, steps, st, cfg, inbox);
+	return n_freq == 0   ? launch_dyst<1, 0>(T, g, dc, n_freq, queue, steps, st, cfg, inbox)
+	       : n_freq <= 4 ? launch_dyst<1, 1>(T, g, dc, n_freq, queue, steps, st, cfg, inbox)
+	                     : launch_dyst<1, 2>(T, g, dc, n_freq, queue, steps, st, cfg, inbox);
 }
-

@@ -110,8 +110,10 @@ struct Request {
  * device's throughput.  The figures are B200 measurements of the mixed
  * kernels (analytic, numerical); they only size windows and never change a
  * result. */
-constexpr double STEP_LATENCY_S[2] = {1.5e-6, 9e-6};
-constexpr double STEP_COST_S[2] = {1.0 / 4.5e10, 1.0 / 1.4e10};
+constexpr double STEP_LATENCY_S[2] = {1.5e-6, 0.75e-6};
+constexpr double STEP_COST_S[2] = {1.0 / 4.5e10, 1.0 / 4e10};
+/* rays of the numerical kernel an SM holds at once: 12 warps of 8 */
+constexpr unsigned NUM_RAYS_PER_SM = 96;
 constexpr double MIN_ITER_S = 0.05;
 
 /* steps of one ray per interval: the analytic cap |dt|/n_sub
@@ -249,8 +251,7 @@ release(Server *S, Request *r)
  * time on their two streams.  Each launch sizes its grid to its SM count,
  * so with both kinds in flight neither grid takes the whole device and the
  * other kind's launch does not wait for it to drain.  While the numerical
- * renders' rays fit on at most half the SMs at once (2 blocks of 256 per
- * SM), they get the SMs that hold them all: their windows were sized for
+ * renders' rays fit on at most half the SMs at once, they get the SMs that hold them all: their windows were sized for
  * rays that run at once.  Otherwise the SMs are split by the kinds'
  * estimated work this iteration. */
 void
@@ -260,13 +261,13 @@ split_sms(const Server *S, const unsigned long long *total, int *ana_sms, int *n
 	double work[2] = {0.0, 0.0};
 	for(const Request *r : S->inflight)
 		work[r->p.spacetime == GRAY_ST_NUMERICAL ? 1 : 0] += r->window * interval_s(r);
-	unsigned long long blocks = 0;
+	unsigned long long need = 0; /* SMs */
 	for(int g = NUM_GROUP; g < GROUPS; ++g)
-		blocks += (total[g] + 255) / 256;
+		need += (total[g] + NUM_RAYS_PER_SM - 1) / NUM_RAYS_PER_SM;
 	*ana_sms = *num_sms = sms;
 	if(work[0] <= 0.0 || work[1] <= 0.0 || sms < 2)
 		return;
-	int n = (int)std::min<unsigned long long>((blocks + 1) / 2, (unsigned long long)sms);
+	int n = (int)std::min<unsigned long long>(need, (unsigned long long)sms);
 	if(n > sms / 2)
 		n = (int)std::lround(sms * work[1] / (work[0] + work[1]));
 	n = std::max(1, std::min(sms - 1, n));
@@ -390,7 +391,8 @@ iterate(Server *S, std::vector<Request *> &fresh)
 			dc.block = 256;
 			dc.sms = num_sms;
 			e = launch_dyst_mixed_table(T, c->grid->gp, g - NUM_GROUP, q, S->d_steps + g,
-			                            S->s[1], dc);
+			                            S->s[1], dc,
+			                            dyst_between(c->grid->gp, &S->h_tab[start[g]], count[g]));
 		} else {
 			e = launch_mixed_table(T, g, q, S->d_steps + g, S->s[0], cfg,
 			                       count[g] == 1 ? &S->h_tab[start[g]] : nullptr);

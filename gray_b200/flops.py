@@ -33,6 +33,12 @@ FP64 kernel (gray_b200/csrc/kernels_fp64.cu), per call:
   RK4             per component 2 + 2 + 2 + 6 = 12, plus 2 scalars
   step control    16 + 4 for the integer-tick arithmetic
 
+Numerical kernel (gray_b200/csrc/kernels_dyst.cu), per in-box step:
+  RHS             per level read 8 corners x (40 FMA + the four rows'
+                  weighting) = 8 x (80 + 8); u^a u^b 16, weights 15, three
+                  axes 9, acceleration 8
+  RK4 + Kahan     16 per component, 8 components
+
 The reference's own comments count the same KS RHS as about 205 FLOP
 (KS.cl:310-374), counting its divides the same way.
 """
@@ -48,6 +54,10 @@ def fp64_per_step(n_freq, transfer=True):
     nd = 8 + 2 * n_freq
     rhs = 196 + ((49 + 5 * n_freq) if (transfer and n_freq) else 0)
     return 4 * rhs + 12 * nd + 2 + 20
+
+
+def numerical_per_step(levels):
+    return 4 * (levels * 8 * 88 + 48) + 16 * 8 + 3
 
 
 def state_bytes_per_ray(n_freq):
