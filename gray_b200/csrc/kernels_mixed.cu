@@ -911,7 +911,25 @@ launch_nf(const MixedTable &T, const MixedRender &R1, unsigned int *queue,
 	int block = cfg.block > 0 ? cfg.block : maxb;
 	if(block > maxb || block % 32)
 		return cudaErrorInvalidValue;
+	/* few rays: smaller blocks, down to one warp, until every SM has a warp
+	 * and every scheduler one before any has two.  A lone warp's step takes
+	 * 1,260 cycles of dependent latency, and two on one scheduler half as
+	 * long again while others idle: 64^2 rays with 4 frequencies took
+	 * 62.9 ms in 256-thread blocks and take 45.8 ms */
+	const int sms = cfg.sms > 0 ? cfg.sms : 148;
+	const unsigned long long warps = (T.total + 32 * Lanes<V>::N - 1) / (32 * Lanes<V>::N);
+	if(warps < (unsigned long long)sms * (block / 32))
+		block = 32 * (int)((warps + sms - 1) / sms);
 	int per_sm = cfg.blocks_per_sm;
+	/* one render: 128 threads at most.  A block's warps drain together at the end of the
+	 * queue, and with 256 the last ones hold eight warps' registers (512 x
+	 * 384 rays over one interval 4.68 ms, in 128 4.24; 1024^2 rays 224.7
+	 * and 223.0; a batch of 24 renders 1% slower).  As many warps stay
+	 * resident per SM. */
+	if(UNI && block > 128) {
+		per_sm *= (block + 127) / 128;
+		block = 128;
+	}
 	int occ = 0;
 	cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
 		&occ, mixed_kernel<NF, V, ROLLED, UNI>, block, 0);
@@ -920,7 +938,7 @@ launch_nf(const MixedTable &T, const MixedRender &R1, unsigned int *queue,
 	if(per_sm <= 0 || per_sm > occ)
 		per_sm = occ > 0 ? occ : 1;
 	const unsigned long long rays_per_block = (unsigned long long)block * Lanes<V>::N;
-	long long want = (long long)per_sm * (cfg.sms > 0 ? cfg.sms : 148);
+	long long want = (long long)per_sm * sms;
 	long long need = (long long)((T.total + rays_per_block - 1) / rays_per_block);
 	unsigned grid = (unsigned)(want < need ? want : need);
 	if(grid == 0)
