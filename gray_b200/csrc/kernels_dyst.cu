@@ -89,15 +89,20 @@ struct DystConst {
 /* Fractional logical coordinate on a fisheye axis, with the cell found
  * exactly against the node table: the FP32 map only gives the first guess,
  * node comparisons settle it (the answer depends on x and the table alone).
- * cell: an interior cell's x0, x1, 1/(x1 - x0), i; x0 > x1 outside. */
+ * cell: x0, x1, 1/(x1 - x0), i of the cell; past either end the range in
+ * which x is clamped there, with 0 for 1/(x1 - x0). */
 __device__ __forceinline__ float
 axis_search(const float *nd, int n, float x, float Bf, float iAf, float4 &cell)
 {
-	cell = make_float4(INFINITY, -INFINITY, 0.0f, 0.0f);
-	if(!(x >= __ldg(nd)))
-		return 0.0f;              /* before the first node (or NaN): clamp-to-edge */
-	if(x >= __ldg(nd + n - 1))
-		return (float)(n - 1);    /* at or past the last node */
+	const float first = __ldg(nd), last = __ldg(nd + n - 1);
+	if(!(x >= first)) {               /* before the first node (or NaN): clamp-to-edge */
+		cell = make_float4(-INFINITY, first, 0.0f, 0.0f);
+		return 0.0f;
+	}
+	if(x >= last) {                   /* at or past the last node */
+		cell = make_float4(last, INFINITY, 0.0f, (float)(n - 1));
+		return (float)(n - 1);
+	}
 	float ax = fabsf(x);
 	float as = 0.69314718f * lg2_a(ax + sqrt_a(fmaf(ax, ax, 1.0f)));   /* asinh|x| */
 	float cb = as > 0.0f ? ex2_a(0.33333334f * lg2_a(as)) : 0.0f;       /* cbrt     */
@@ -436,7 +441,7 @@ enter_cell(const GridParams &g, const DystConst &dc, Axis &A, Cell<RT> &C, int l
 				const int n = m == 1 ? g.nx : m == 2 ? g.ny : g.nz;
 				float4 cell;
 				uu = axis_search(g.nodes_f[m - 1], n, xs, dc.B[m - 1], dc.iA[m - 1], cell);
-				A.x0 = cell.x;
+				A.x0 = cell.z > 0.0f ? cell.x : 0.0f;
 				A.inv = cell.z;
 				A.ci = cell.w;
 				A.xa = cell.x;

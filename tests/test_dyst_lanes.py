@@ -1,8 +1,9 @@
-"""The mixed numerical kernel's lanes, cells and level codes: where a ray's
-cell, box side or time levels change, and at the edges of its groups."""
+"""The numerical kernels' lanes, cells and level codes: where a ray's cell,
+box side or time levels change, and at the edges of its groups."""
 import numpy as np
 import pytest
 
+import oracle as O
 from gray_b200 import api
 
 BOX = 40.0
@@ -86,3 +87,32 @@ def test_chunked_flat_steps_keep_every_step(ctx):
         b.close()
         for r in rs:
             r.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_freq", [0, 5])
+@pytest.mark.parametrize("shape,levels,physics,cfg", [
+    ((1, 1), (0.0, 0.0), True, dict(r_obs=45.0, dt_dump=-7.0, n_dump=2)),     # flat chunks, then the box
+    ((9, 1), (0.0, 0.0), False, dict(r_obs=44.0, dt_dump=-3.0, n_dump=3)),    # clamped past the last node
+    ((13, 5), (-3.0, 0.0), False, dict(n_dump=3)),                            # eight lanes per ray
+    ((7, 3), (-3.0, -1.0), True, dict(n_dump=3, r_obs=41.0)),                 # time clamped at both ends
+])
+def test_fp64_lanes_match_oracle(ctx, n_freq, shape, levels, physics, cfg):
+    """Each lane's operations are the oracle's in its order: the geodesic
+    columns and step counts are equal, the transfer within 1e-10 (its exp,
+    log and cbrt are not glibc's)."""
+    n = 20
+    t1, t2 = levels
+    lv = [O.boosted_ks_grid(n, -BOX, BOX, t, a=0.7, v=0.3, axis=1) for t in levels]
+    grid = api.make_grid(n, -BOX, BOX, t1, t2, physics=physics)
+    for k in (0, 1):
+        ctx.load_spacetime(grid, lv[k], k)
+    og = O.Grid(lv if t1 != t2 else lv[:1], [t1, -BOX, -BOX, -BOX, t2, BOX, BOX, BOX],
+                physics=physics)
+    c = dict(BASE, **dict(cfg, n_width=shape[0], n_height=shape[1], nu=NU[:n_freq],
+                          precision=api.PREC_FP64))
+    got, steps = state(ctx, c)
+    ref, _, osteps = O.dyst_trace(c, og, np.arange(shape[0] * shape[1]))
+    assert steps == osteps.sum()
+    assert np.array_equal(got[:8].T, ref[:, :8])
+    assert np.all(np.abs(got[8:].T - ref[:, 8:]) <= 1e-10 * np.abs(ref[:, 8:]))
