@@ -71,7 +71,6 @@ struct gray_ctx {
 	std::map<int, Render *> renders;
 	int next_id = 1;
 	Grid *grid = nullptr;
-	int evolve64_block = 128;
 	/* default plan (GRAY_PLAN_ESTIMATE): one ray per thread, 256-thread
 	 * blocks -- the shape the measuring planner picks on B200 for the
 	 * analytic torus renders */

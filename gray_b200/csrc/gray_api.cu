@@ -567,8 +567,8 @@ evolve_interval(gray_ctx *c, Render *r, double t, double target, uint64_t n_sub)
 		return run_mixed(c, r, t, dt, 1, (long long)n_sub);
 	}
 	if(r->desc.precision == GRAY_PREC_FP64) {
-		CK(launch_evolve64(r->p, r->d_data, r->d_info, dt, (long long)n_sub,
-		                   r->d_steps, c->stream, c->evolve64_block));
+		CK(launch_evolve64(r->p, r->d_data, r->d_info, t, dt, 1, (long long)n_sub,
+		                   r->d_steps, c->stream));
 		return GRAY_OK;
 	}
 	return run_mixed(c, r, t, dt, 1, (long long)n_sub);
@@ -606,6 +606,9 @@ evolve_all_impl(gray_ctx *c, Render *r)
 		st = run_mixed(c, r, d.t_init, d.dt_dump, (long long)d.n_dump, (long long)d.n_sub);
 		if(st)
 			return st;
+	} else if(r->p.spacetime == GRAY_ST_KERR && d.n_dump > 1) {
+		CK(launch_evolve64(r->p, r->d_data, r->d_info, d.t_init, d.dt_dump,
+		                   (long long)d.n_dump, (long long)d.n_sub, r->d_steps, c->stream));
 	} else {
 		/* sim-org/gray.c:248-257 */
 		for(uint64_t i = 0; i < d.n_dump;) {

@@ -74,10 +74,11 @@ void gray_internal_make_params(const gray_render_desc *d, RenderParams *p);
 /* ---- launchers (one per translation unit) ---- */
 cudaError_t launch_icond64(const RenderParams &p, double *data, double *info,
                            cudaStream_t st);
+/* n_dump intervals of length dt_dump from t_init; of one interval dt_dump is
+ * its exact length */
 cudaError_t launch_evolve64(const RenderParams &p, double *data, double *info,
-                            double dt, long long n_sub,
-                            unsigned long long *steps, cudaStream_t st,
-                            int block);
+                            double t_init, double dt_dump, long long n_dump,
+                            long long n_sub, unsigned long long *steps, cudaStream_t st);
 cudaError_t launch_kdown64(const RenderParams &p, const double *data, double *k,
                            cudaStream_t st);
 cudaError_t launch_getuu64(const RenderParams &p, const double *data, double *info,
