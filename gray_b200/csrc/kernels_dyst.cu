@@ -18,7 +18,7 @@
  * 1965 MHz, one ray per thread before and four lanes now: 512^2 rays at 200 M
  * on a 128^3 grid 530 -> 197 ms (1.48e10 -> 3.99e10 ray-steps/s), 97 x 72
  * rays on a 256^3 grid 243 -> 22.8 ms, 160 x 120 rays between two levels
- * with four frequencies 44.6 -> 17.8 ms; outputs bit-identical.  The pairs
+ * with four frequencies 47.3 -> 14.3 ms; outputs bit-identical.  The pairs
  * are kept as 64-bit values: as float2 the compiler repacked the cell at
  * every RHS (247 instructions, 301 ms).  At 128 registers and 16 warps the
  * large render took 196 ms but the spills cost small ones 17% (20.3 ms
@@ -28,7 +28,13 @@
  * four per level.
  *
  * Thermal transfer: lanes 0 and 3 also hold their rows of g (for k_t and
- * k_z), lane 1 rho, and the frequencies are divided among the ray's lanes.
+ * k_z), lane 1 rho.  Emission and absorption at a stage depend on the
+ * geodesic alone, so the four stages are walked first and then lane m
+ * evaluates stage m, one frequency per pass (two with eight lanes); only
+ * e^-tau chains the stages, through one shuffle.  With a frequency per lane
+ * instead, 200 x 160 rays between two levels took 28.1 ms for one frequency
+ * (now 19.0) and 160 x 120 rays 17.5 ms for four (14.3); eight frequencies in
+ * one level, where no lane idled, 14.7 (18.0).
  *
  * Grid layout: per time level float [nz][ny][nx][GRAY_NSTRIDE] with the
  * fields of one grid point contiguous (Gamma 0..39, g 40..49, rho 50, pad).
@@ -148,79 +154,84 @@ exp_f(float x)
  * stay FP64, the special functions of O(1) arguments (exp, log, cbrt,
  * sqrt) take the FP32 approximate instructions, and everything that
  * depends only on the render is a ThermalFast constant.  Same formulas and
- * branches as the FP64 kernels; agreement to ~1e-6 relative.  N: the
- * frequencies of this lane. */
-template <int N>
-__device__ __forceinline__ void
-rt_rhs_fast(const ThermalFast &t, const double *nu_hz, double kt, double kz, double ne,
-            const double *tau, double *dI, double *dtau)
+ * branches as the FP64 kernels; agreement to ~1e-6 relative. */
+struct RayFrame { /* what the frequencies of a ray at one event share */
+	double shift, ish2, nus, inus, ne;
+	bool syn;
+};
+
+__device__ __forceinline__ RayFrame
+ray_frame(const ThermalFast &t, double kt, double kz, double ne)
 {
 	const double EPS = GRAY_EPSILON;
-	const double shift = -kt;
-	const float bkcos = (float)(kz * t.b) * rcp_a((float)(shift * t.b + EPS));
-	const double ish2 = rcp64(fma(shift, shift, EPS));
+	RayFrame r;
+	r.ne = ne;
+	r.shift = -kt;
+	const float bkcos = (float)(kz * t.b) * rcp_a((float)(r.shift * t.b + EPS));
+	r.ish2 = rcp64(fma(r.shift, r.shift, EPS));
 	/* synchrotron frequency: nu_s = knus sin(theta), zero along the field */
-	double nus = 0.0, inus = 0.0;
-	const bool syn = t.syn && bkcos > -1.0f && bkcos < 1.0f;
-	if(syn) {
-		nus = t.knus * (double)sqrt_a(fmaf(-bkcos, bkcos, 1.0f));
-		inus = rcp64(nus + EPS);
+	r.nus = r.inus = 0.0;
+	r.syn = t.syn && bkcos > -1.0f && bkcos < 1.0f;
+	if(r.syn) {
+		r.nus = t.knus * (double)sqrt_a(fmaf(-bkcos, bkcos, 1.0f));
+		r.inus = rcp64(r.nus + EPS);
 	}
-	const double ne2 = ne * ne;
-#pragma unroll
-	for(int i = 0; i < N; ++i) {
-		const double nu = nu_hz[i] * shift;
-		/* rt.cl:80-93 */
-		const double f2 = nu * t.kf2;
-		double B;
-		if(f2 > 1e-5) {
-			double em1;
-			if(f2 < 0.3) /* e^f2 - 1 by its series: no cancellation */
-				em1 = f2 * fma(f2, fma(f2, fma(f2, fma(f2, fma(f2, fma(f2,
-				      1.0 / 5040, 1.0 / 720), 1.0 / 120), 1.0 / 24), 1.0 / 6), 0.5), 1.0);
-			else if(f2 < 80.0)
-				em1 = (double)exp_f((float)f2) - 1.0;
-			else
-				em1 = exp(f2);
-			B = t.kB * (nu * nu) * nu / em1;
-		} else {
-			B = t.kB2 * (nu * nu) * rcp64(fma(f2, fma(f2, 1.0 / 6, 0.5), 1.0));
-		}
-		/* rt.cl:95-143 bremsstrahlung */
-		const double y = nu * t.ky;
-		double Lff = 0.0;
-		if(y < 80.0) {
-			const float yf = (float)(y + EPS);
-			const float sy = sqrt_a((float)y);
-			double G;
-			if(t.xg > 1.0)
-				G = y > 1.0 ? t.g1 / (double)sy
-				            : t.g2 * (t.g3 - 0.6931471805599453 * (double)lg2_a(yf));
-			else if(t.xg * y > 1.0)
-				G = t.g5 * rcp64(t.sxg * (double)sy);
-			else if(y > t.sxg)
-				G = 1.0;
-			else {
-				G = t.g2 * (t.g4 + 0.6931471805599453 *
-				                      (double)(lg2_a((float)t.sxg) - lg2_a(yf)));
-				G = G > EPS ? G : EPS;
-			}
-			Lff = (t.kff * ne2) * G * rcp64(fma(t.sqte, (double)exp_f((float)y), EPS));
-		}
-		/* rt.cl:145-170 synchrotron */
-		double Lsyn = 0.0;
-		if(syn) {
-			double x = nu * inus;
-			x = x < 1e30 ? x : 1e30; /* e^-cbrt(x) is 0 long before */
-			const float xf = (float)x;
-			const float cx = ex2_a(0.33333334f * lg2_a(xf));
-			const double xx = (double)sqrt_a(xf) + 1.88774862536 * (double)sqrt_a(cx);
-			Lsyn = t.ksyn * (xx * xx) * (double)exp_f(-cx) * (ne * nus);
-		}
-		const double L = Lsyn + Lff;
-		dI[i]   = -L * (double)exp_f(-(float)tau[i]) * ish2;
-		dtau[i] = -L * shift * rcp64(B + EPS);
+	return r;
+}
+
+/* L_nu at the event, and B_nu */
+__device__ __forceinline__ double
+emissivity(const ThermalFast &t, const RayFrame &r, double nu_hz, double &B)
+{
+	const double EPS = GRAY_EPSILON;
+	const double nu = nu_hz * r.shift;
+	/* rt.cl:80-93 */
+	const double f2 = nu * t.kf2;
+	if(f2 > 1e-5) {
+		double em1;
+		if(f2 < 0.3) /* e^f2 - 1 by its series: no cancellation */
+			em1 = f2 * fma(f2, fma(f2, fma(f2, fma(f2, fma(f2, fma(f2,
+			      1.0 / 5040, 1.0 / 720), 1.0 / 120), 1.0 / 24), 1.0 / 6), 0.5), 1.0);
+		else if(f2 < 80.0)
+			em1 = (double)exp_f((float)f2) - 1.0;
+		else
+			em1 = exp(f2);
+		B = t.kB * (nu * nu) * nu / em1;
+	} else {
+		B = t.kB2 * (nu * nu) * rcp64(fma(f2, fma(f2, 1.0 / 6, 0.5), 1.0));
 	}
+	/* rt.cl:95-143 bremsstrahlung */
+	const double y = nu * t.ky;
+	double Lff = 0.0;
+	if(y < 80.0) {
+		const float yf = (float)(y + EPS);
+		const float sy = sqrt_a((float)y);
+		double G;
+		if(t.xg > 1.0)
+			G = y > 1.0 ? t.g1 / (double)sy
+			            : t.g2 * (t.g3 - 0.6931471805599453 * (double)lg2_a(yf));
+		else if(t.xg * y > 1.0)
+			G = t.g5 * rcp64(t.sxg * (double)sy);
+		else if(y > t.sxg)
+			G = 1.0;
+		else {
+			G = t.g2 * (t.g4 + 0.6931471805599453 *
+			                      (double)(lg2_a((float)t.sxg) - lg2_a(yf)));
+			G = G > EPS ? G : EPS;
+		}
+		Lff = (t.kff * (r.ne * r.ne)) * G * rcp64(fma(t.sqte, (double)exp_f((float)y), EPS));
+	}
+	/* rt.cl:145-170 synchrotron */
+	double Lsyn = 0.0;
+	if(r.syn) {
+		double x = nu * r.inus;
+		x = x < 1e30 ? x : 1e30; /* e^-cbrt(x) is 0 long before */
+		const float xf = (float)x;
+		const float cx = ex2_a(0.33333334f * lg2_a(xf));
+		const double xx = (double)sqrt_a(xf) + 1.88774862536 * (double)sqrt_a(cx);
+		Lsyn = t.ksyn * (xx * xx) * (double)exp_f(-cx) * (r.ne * r.nus);
+	}
+	return Lsyn + Lff;
 }
 
 /* ------------------------------------------------------------ the kernel */
@@ -590,11 +601,6 @@ dyst_accel(const GridParams &g, const DystConst &dc, Axis &A, Cell<RT> &C, int l
 		kn[0] = __shfl_sync(FULL, Km, 0, L);
 		kn[1] = __shfl_sync(FULL, Km, 3, L);
 		kn[2] = __shfl_sync(FULL, Km, 1, L);
-		if(!in) { /* flat space, empty */
-			kn[0] = -u0;
-			kn[1] = u3;
-			kn[2] = 0.0f;
-		}
 	}
 	return fmaf(G0, us, -G);
 }
@@ -650,6 +656,45 @@ final_uu(const GridParams &g, double q0, double q1, double q2, double q3, double
 	return dyst_getuu64(g, s);
 }
 
+/* RK4 of a ray's (I, tau) over a step of hs, given on lane m the frame of
+ * stage m.  Frequency f is kept by lane (f / LV) % 4 of half f % LV. */
+template <int LV, int FPL>
+__device__ __forceinline__ void
+transfer(const MixedRender &c, int nf, unsigned gmask, int lane, double hs, float kt, float kz,
+         float ne, double *I, double *tau)
+{
+	const int m = lane & 3, l = LV == 2 ? (lane >> 2) & 1 : 0;
+	const ThermalFast &t = c.tf;
+	const RayFrame r = ray_frame(t, kt, kz, ne);
+	const double h6 = hs / 6.0, cd = m == 3 ? hs : 0.5 * hs;
+#pragma unroll
+	for(int i = 0; i < FPL; ++i)
+#pragma unroll 1
+		for(int q = 0; q < 4; ++q) {
+			const int f = LV * (4 * i + q) + l;
+			if(LV * (4 * i + q) >= nf)
+				break;
+			double B;
+			const double nL = -emissivity(t, r, c.nu_hz[f < nf ? f : 0], B);
+			const double dt = nL * r.shift * rcp64(B + GRAY_EPSILON);
+			const double t0 = __shfl_sync(gmask, tau[i], q, 4);
+			const double before = __shfl_up_sync(gmask, dt, 1, 4);
+			const double st = m ? fma(cd, before, t0) : t0;
+			const double dI = nL * (double)exp_f(-(float)st) * r.ish2;
+			double sI = __shfl_sync(gmask, dI, 0, 4), sT = __shfl_sync(gmask, dt, 0, 4);
+#pragma unroll
+			for(int k = 1; k < 4; ++k) {
+				const double w = k < 3 ? 2.0 : 1.0;
+				sI = fma(w, __shfl_sync(gmask, dI, k, 4), sI);
+				sT = fma(w, __shfl_sync(gmask, dt, k, 4), sT);
+			}
+			if(m == q && f < nf) {
+				I[i] = fma(h6, sI, I[i]);
+				tau[i] = fma(h6, sT, tau[i]);
+			}
+		}
+}
+
 constexpr int DYST_BLOCK = 128;
 
 /* LV: the time levels a ray's lanes hold; FPL: frequencies
@@ -663,8 +708,8 @@ dyst_mixed_kernel(const MixedTable T, const __grid_constant__ GridParams g, cons
 {
 	constexpr int L = 4 * LV;   /* lanes per ray */
 	constexpr bool RT = FPL > 0;
-	/* stages unrolled: 197 ms against 225 on the 512^2 render; with the
-	 * transfer one body measures faster (17.5 ms against 20.4) */
+	/* stages unrolled: 197 ms against 225 on the 512^2 render; beside the
+	 * transfer one body (its registers are short) */
 	constexpr int STAGES = RT ? 1 : 4;
 	constexpr int NR = RT ? FPL : 1;
 	const unsigned FULL = 0xffffffffu;
@@ -678,10 +723,12 @@ dyst_mixed_kernel(const MixedTable T, const __grid_constant__ GridParams g, cons
 	A.x0 = A.inv = A.ci = A.xb = 0.0f;
 
 	float xh = 0.0f, xl = 0.0f, uh = 0.0f, ul = 0.0f; /* x^m, u^m: high and low parts */
-	double I[NR], tau[NR], nu[NR];
+	/* (I, tau) of the frequencies this lane keeps: own(0), own(1) */
+	auto own = [&](int i) { return LV * (4 * i + m) + (sub >> 2); };
+	double I[NR], tau[NR];
 #pragma unroll
 	for(int i = 0; i < NR; ++i)
-		I[i] = tau[i] = nu[i] = 0.0;
+		I[i] = tau[i] = 0.0;
 	unsigned ray = 0;
 	int dump = 0, h = 0, dh_step = 0, n = 0;
 	float dtn = 0.0f;
@@ -722,10 +769,9 @@ dyst_mixed_kernel(const MixedTable T, const __grid_constant__ GridParams g, cons
 						if constexpr(RT) {
 #pragma unroll
 							for(int i = 0; i < FPL; ++i) {
-								const int f = sub + i * L < nf ? sub + i * L : 0;
+								const int f = own(i) < nf ? own(i) : 0;
 								I[i] = c->data[(8 + f) * c->n_rays + ray];
 								tau[i] = c->data[(8 + nf + f) * c->n_rays + ray];
-								nu[i] = c->nu_hz[f];
 							}
 						}
 						dump = c->dump_begin - 1;
@@ -768,9 +814,9 @@ dyst_mixed_kernel(const MixedTable T, const __grid_constant__ GridParams g, cons
 				if constexpr(RT) {
 #pragma unroll
 					for(int i = 0; i < FPL; ++i)
-						if(sub + i * L < nf) {
-							c->data[(8 + sub + i * L) * c->n_rays + ray] = I[i];
-							c->data[(8 + nf + sub + i * L) * c->n_rays + ray] = tau[i];
+						if(own(i) < nf) {
+							c->data[(8 + own(i)) * c->n_rays + ray] = I[i];
+							c->data[(8 + nf + own(i)) * c->n_rays + ray] = tau[i];
 						}
 				}
 				if(sub == 0)
@@ -798,11 +844,11 @@ dyst_mixed_kernel(const MixedTable T, const __grid_constant__ GridParams g, cons
 		const float h6 = hs * (1.0f / 6.0f);
 
 		/* flat space through the whole step (physics mode outside the box):
-		 * no field enters, u is constant.  Not asked where the last step
-		 * found every ray inside. */
+		 * no field enters, u is constant, nothing emits.  Not asked where the
+		 * last step found every ray inside. */
 		bool out = false, in0 = true, in = true; /* out: this ray, all step long */
 		bool flat = false;
-		if(!RT && g.physics && !quiet) {
+		if(g.physics && !quiet) {
 			const float lo = g.box[m], hi = g.box[m + 4];
 			auto outside = [&](float x) {
 				unsigned b = __ballot_sync(FULL, m > 0 && !(x >= lo && x <= hi));
@@ -822,18 +868,11 @@ dyst_mixed_kernel(const MixedTable T, const __grid_constant__ GridParams g, cons
 			              cnt))
 				continue;
 		} else {
-			float kn[3];
+			float kn[3], kt = 0.0f, kz = 0.0f, ne = 0.0f; /* stage m's */
 			bool all = true;
 			quiet = true;
-			double Is[NR], ts[NR], dI[NR], dtau[NR], st[NR];
-			const double hsd = (double)dh * dtnd;
 			sx = su = 0.0f;
 			float x = xh, u = uh;
-#pragma unroll
-			for(int i = 0; i < NR; ++i) {
-				st[i] = tau[i];
-				Is[i] = ts[i] = 0.0;
-			}
 #pragma unroll STAGES
 			for(int s = 0; s < 4; ++s) {
 				kx = u;
@@ -842,20 +881,14 @@ dyst_mixed_kernel(const MixedTable T, const __grid_constant__ GridParams g, cons
 				quiet = quiet && all;
 				in0 = s == 0 ? in : in0;
 				ku = in ? ku : 0.0f;
+				if(RT && s == m) {
+					/* flat space, empty, outside */
+					kt = in ? kn[0] : -1.0f;
+					kz = in ? kn[1] : 0.0f;
+					ne = in ? kn[2] : 0.0f;
+				}
 				const float wg = (s == 1 || s == 2) ? 2.0f : 1.0f;
 				const float cg = s < 2 ? hh : hs;
-				if constexpr(RT) {
-					const double wd = wg, cd = s < 2 ? 0.5 * hsd : hsd;
-					if(step)
-						rt_rhs_fast<NR>(c->tf, nu, (double)kn[0], (double)kn[1],
-						                (double)kn[2], st, dI, dtau);
-#pragma unroll
-					for(int i = 0; i < NR; ++i) {
-						Is[i] = s == 0 ? dI[i] : fma(wd, dI[i], Is[i]);
-						ts[i] = s == 0 ? dtau[i] : fma(wd, dtau[i], ts[i]);
-						st[i] = fma(cd, dtau[i], tau[i]);
-					}
-				}
 				if(s < 3) { /* k4 stays in kx, ku for the update */
 					sx = s == 0 ? kx : fmaf(wg, kx, sx);
 					su = s == 0 ? ku : fmaf(wg, ku, su);
@@ -865,13 +898,9 @@ dyst_mixed_kernel(const MixedTable T, const __grid_constant__ GridParams g, cons
 			}
 			quiet = quiet && __all_sync(FULL, !out);
 			if constexpr(RT) {
-				if(step) {
-#pragma unroll
-					for(int i = 0; i < NR; ++i) {
-						I[i] = fma(hsd / 6.0, Is[i], I[i]);
-						tau[i] = fma(hsd / 6.0, ts[i], tau[i]);
-					}
-				}
+				const double hsd = (double)dh * dtnd;
+				if(step) /* uniform over a ray's lanes */
+					transfer<LV, FPL>(*c, nf, gmask, lane, hsd, kt, kz, ne, I, tau);
 			}
 		}
 		/* compensated update, value = hi - lo */

@@ -275,6 +275,50 @@ flat_chunk64(const GridParams &g, int m, bool step, double x, double dx, int lef
 	return todo == INT_MAX ? 0 : todo;
 }
 
+/* RK4 of a ray's (I, tau) over a step of hs (rt.cl:185-198 with getflow() of
+ * flow.cl:36-58), given on lane m k_t, k_z and n_e at stage m: what a stage
+ * emits and absorbs depends on the geodesic alone, so lane m evaluates stage
+ * m, a frequency per pass (two with eight lanes), and only e^-tau chains the
+ * stages.  Frequency f is kept by lane (f / LV) % 4 of half f % LV. */
+template <int LV, int FPL>
+__device__ __forceinline__ void
+transfer64(const RenderParams &p, int lane, double hs, double h6, double kt, double kz, double ne,
+           double *I, double *tau)
+{
+	const unsigned FULL = 0xffffffffu;
+	const int m = lane & 3, l = LV == 2 ? (lane >> 2) & 1 : 0;
+	const double shift = -kt;
+	const double bkcos = (kz * p.flow_b) / (shift * p.flow_b + thermal::EPS);
+	const double cd = m == 3 ? hs : 0.5 * hs;
+#pragma unroll
+	for(int i = 0; i < FPL; ++i)
+#pragma unroll 1
+		for(int q = 0; q < 4; ++q) {
+			const int f = LV * (4 * i + q) + l;
+			if(LV * (4 * i + q) >= p.n_freq)
+				break;
+			const double nu = p.nu[f < p.n_freq ? f : 0] * shift;
+			const double B = thermal::B_Planck(nu, p.flow_te);
+			const double nL = -(thermal::L_j_syn(p.th, p.m_adm, nu, p.flow_te, ne, p.flow_b, bkcos) +
+			                    thermal::L_j_ff(p.th, p.m_adm, nu, p.flow_te, ne));
+			const double dt = nL * shift / (B + thermal::EPS);
+			const double t0 = __shfl_sync(FULL, tau[i], q, 4);
+			const double before = __shfl_up_sync(FULL, dt, 1, 4);
+			const double st = m ? fma(cd, before, t0) : t0;
+			const double dI = nL * exp(-st) / (shift * shift + thermal::EPS);
+			double kI[4], kT[4];
+#pragma unroll
+			for(int k = 0; k < 4; ++k) {
+				kI[k] = __shfl_sync(FULL, dI, k, 4);
+				kT[k] = __shfl_sync(FULL, dt, k, 4);
+			}
+			if(m == q && f < p.n_freq) {
+				I[i] = fma(h6, fma(2.0, kI[1] + kI[2], kI[0]) + kI[3], I[i]);
+				tau[i] = fma(h6, fma(2.0, kT[1] + kT[2], kT[0]) + kT[3], tau[i]);
+			}
+		}
+}
+
 constexpr int BLOCK64 = 64;
 
 /* driver.cl:69-108 on the numerical spacetime over one dump interval of
@@ -285,7 +329,7 @@ constexpr int BLOCK64 = 64;
  * transfer the emissivities' exp, log and cbrt.  Measured, one ray per thread
  * before and four (two levels: eight) lanes now: 256 x 200 rays in one level
  * 65.5 -> 13.0 ms, 64 x 48 rays between two levels 92.1 -> 2.8 ms, with one
- * frequency 130.5 -> 14.6 ms.  Before, every RHS converted 320 floats a ray
+ * frequency 130.5 -> 8.5 ms (14.6 with a frequency per lane).  Before, every RHS converted 320 floats a ray
  * to double and searched each axis with cbrt and asinh. */
 template <int LV, int FPL>
 __global__ void __launch_bounds__(BLOCK64, 4)
@@ -321,23 +365,22 @@ dyst_evolve64_kernel(const __grid_constant__ RenderParams p, const __grid_consta
 			for(int k = 0; k < 4; ++k)
 				C.W[c][k] = 0.0f;
 	}
-	double x = 0.0, u = 0.0, I[NR], tau[NR], nu[NR];
+	/* (I, tau) of the frequencies this lane keeps: own(0), own(1) */
+	auto own = [&](int i) { return LV * (4 * i + m) + (sub >> 2); };
+	double x = 0.0, u = 0.0, I[NR], tau[NR];
 	if(mine) {
 		x = data[m * nr + r];
 		u = data[(4 + m) * nr + r];
 	}
 #pragma unroll
 	for(int i = 0; i < NR; ++i) {
-		const int f = sub + i * L < p.n_freq ? sub + i * L : 0;
-		I[i] = tau[i] = nu[i] = 0.0;
+		const int f = own(i) < p.n_freq ? own(i) : 0;
+		I[i] = tau[i] = 0.0;
 		if(RT && mine) {
 			I[i] = data[(8 + f) * nr + r];
 			tau[i] = data[(8 + p.n_freq + f) * nr + r];
-			nu[i] = p.nu[f];
 		}
 	}
-	const thermal::Flow flow = {nu, p.m_adm, p.flow_te, p.flow_b, &p.th};
-
 	const int n = (int)((INT_MAX / n_sub) * n_sub);
 	const double dts = dt / (double)n_sub;
 	const int dh_step = (int)(dyst_getdt64(dts) / dt * (double)n);
@@ -348,7 +391,7 @@ dyst_evolve64_kernel(const __grid_constant__ RenderParams p, const __grid_consta
 		const double hs = ((double)dh * dt) / (double)n, hh = 0.5 * hs;
 		const double h6 = hs / 6.0;
 		bool out = false; /* in flat space all step long */
-		if(!RT && g.physics && !quiet) {
+		if(g.physics && !quiet) {
 			const double lo = (double)g.box[m], hi = (double)g.box[m + 4];
 			auto outside = [&](double q) {
 				const unsigned b = __ballot_sync(FULL, m > 0 && !(q >= lo && q <= hi));
@@ -369,12 +412,7 @@ dyst_evolve64_kernel(const __grid_constant__ RenderParams p, const __grid_consta
 			}
 		}
 		double xq = x, uq = u, kx1 = 0.0, ku1 = 0.0, kx2 = 0.0, ku2 = 0.0, kx = 0.0, ku = 0.0;
-		double st[NR], dI[NR], dtau[NR], I1[NR], I2[NR], t1[NR], t2[NR];
-#pragma unroll
-		for(int i = 0; i < NR; ++i) {
-			st[i] = tau[i];
-			I1[i] = I2[i] = t1[i] = t2[i] = 0.0;
-		}
+		double kt = 0.0, kz = 0.0, ne = 0.0; /* stage m's */
 		quiet = true;
 #pragma unroll STAGES
 		for(int s = 0; s < 4; ++s) {
@@ -382,17 +420,14 @@ dyst_evolve64_kernel(const __grid_constant__ RenderParams p, const __grid_consta
 			bool in = true, all = true;
 			kx = uq;
 			ku = dyst_accel64<LV, RT>(g, A, C, lane, mine && !out, xq, uq, kn, in, all);
-			if(RT && !in) { /* flat space, empty */
-				kn[0] = -__shfl_sync(0xfu << (lane & ~3), uq, 0, 4);
-				kn[1] = __shfl_sync(0xfu << (lane & ~3), uq, 3, 4);
-				kn[2] = 0.0;
-			}
 			in = in && !out;
 			quiet = quiet && all;
 			ku = in ? ku : 0.0;
-			if constexpr(RT) {
-				const double k4[4] = {kn[0], 0.0, 0.0, kn[1]};
-				thermal::rt_rhs<NR>(flow, k4, kn[2], st, dI, dtau);
+			if(RT && s == m) {
+				/* flat space, empty, outside */
+				kt = in ? kn[0] : -1.0;
+				kz = in ? kn[1] : 0.0;
+				ne = in ? kn[2] : 0.0;
 			}
 			const double cg = s < 2 ? hh : hs;
 			if(s == 0) {
@@ -404,31 +439,13 @@ dyst_evolve64_kernel(const __grid_constant__ RenderParams p, const __grid_consta
 			}
 			xq = fma(cg, kx, x);
 			uq = fma(cg, ku, u);
-			if constexpr(RT) {
-#pragma unroll
-				for(int i = 0; i < NR; ++i) {
-					if(s == 0) {
-						I1[i] = dI[i];
-						t1[i] = dtau[i];
-					} else if(s < 3) {
-						I2[i] = s == 1 ? dI[i] : I2[i] + dI[i];
-						t2[i] = s == 1 ? dtau[i] : t2[i] + dtau[i];
-					}
-					st[i] = fma(cg, dtau[i], tau[i]);
-				}
-			}
 		}
 		quiet = quiet && __all_sync(FULL, !out);
 		/* RK4.cl:37-47 */
 		x = fma(h6, fma(2.0, kx2, kx1) + kx, x);
 		u = fma(h6, fma(2.0, ku2, ku1) + ku, u);
-		if constexpr(RT) {
-#pragma unroll
-			for(int i = 0; i < NR; ++i) {
-				I[i] = fma(h6, fma(2.0, I2[i], I1[i]) + dI[i], I[i]);
-				tau[i] = fma(h6, fma(2.0, t2[i], t1[i]) + dtau[i], tau[i]);
-			}
-		}
+		if constexpr(RT)
+			transfer64<LV, FPL>(p, lane, hs, h6, kt, kz, ne, I, tau);
 		++cnt;
 		h += dh;
 	}
@@ -446,9 +463,9 @@ dyst_evolve64_kernel(const __grid_constant__ RenderParams p, const __grid_consta
 		if constexpr(RT) {
 #pragma unroll
 			for(int i = 0; i < NR; ++i)
-				if(sub + i * L < p.n_freq) {
-					data[(8 + sub + i * L) * nr + r] = I[i];
-					data[(8 + p.n_freq + sub + i * L) * nr + r] = tau[i];
+				if(own(i) < p.n_freq) {
+					data[(8 + own(i)) * nr + r] = I[i];
+					data[(8 + p.n_freq + own(i)) * nr + r] = tau[i];
 				}
 		}
 		if(sub == 0)

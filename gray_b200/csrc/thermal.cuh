@@ -107,34 +107,6 @@ L_j_syn(const ThermalConsts &t, double m_adm, double nu, double te, double ne, d
 	return (m_adm * xx * exp(-cbrtx)) * (xx * exp(-log_K2)) * (f * ne * nus);
 }
 
-/* Per-render inputs of the transfer. */
-struct Flow {
-	const double *nu;   /* observed frequencies [NF] (Hz)      */
-	double m_adm, te, b;
-	const ThermalConsts *th;
-};
-
-/* rt.cl:185-198 with getflow() of flow.cl:36-58: k is the covariant
- * photon momentum, tau[NF] the optical depths of the state; writes
- * dI[NF], dtau[NF]. */
-template <int NF>
-__device__ __forceinline__ void
-rt_rhs(const Flow &f, const double k[4], double ne, const double *tau, double *dI,
-       double *dtau)
-{
-	const double shift = -k[0];
-	const double bkcos = (k[3] * f.b) / (shift * f.b + EPS);
-#pragma unroll
-	for(int i = 0; i < NF; ++i) {
-		const double nu = f.nu[i] * shift;
-		const double B_nu = B_Planck(nu, f.te);
-		const double L = L_j_syn(*f.th, f.m_adm, nu, f.te, ne, f.b, bkcos) +
-		                 L_j_ff(*f.th, f.m_adm, nu, f.te, ne);
-		dI[i]   = -L * exp(-tau[i]) / (shift * shift + EPS);
-		dtau[i] = -L * shift / (B_nu + EPS);
-	}
-}
-
 } /* namespace thermal */
 
 #endif /* GRAY_THERMAL_CUH */
