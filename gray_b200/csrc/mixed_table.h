@@ -29,7 +29,7 @@ struct ThermalFast {
 };
 
 struct MixedRender {
-	float  a, aa, rp, risco, eps_stop;
+	float  a, aa, nhaa, rp, risco, eps_stop; /* nhaa = -a^2/2 */
 	float  cdt_scale;          /* 0.01: the step fraction of phys.cl:60-61     */
 	float  kappa, n0_rp15, ihr2_log2e;
 	float  nupow[GRAY_MAX_FREQ];

@@ -8,10 +8,10 @@ every step of the torus workloads; outside it the transfer part is skipped.
 
 Mixed kernel (gray_b200/csrc/kernels_mixed.cu), per call; the geodesic is
 integrated in Hamiltonian form on (x^mu, k_i) with k_t conserved:
-  ks_ham          93   (head 32: radius root, f, df/dr and the explicit
+  ks_ham          92   (head 32: radius root, f, df/dr and the explicit
                         df/dz with 2 rsqrt + 2 rcp; l, L = l^mu k_mu,
                         dL/dr and the force G d_i r + f L (explicit d_i L),
-                        and dx^mu/dl 61)
+                        and dx^mu/dl 60)
   torus_rt        33 + 4 per frequency  (Keplerian flow and shift from
                         k_mu 23; the density in log2, -1.5 lg2 r plus the
                         Gaussian from z/r of the geodesic part, and dtau_0 as
@@ -46,7 +46,7 @@ The reference's own comments count the same KS RHS as about 205 FLOP
 
 def mixed_per_step(n_freq, transfer=True):
     ni = 7 + (n_freq + 1 if n_freq else 0)
-    rhs = 93 + ((33 + 4 * n_freq) if (transfer and n_freq) else 0)
+    rhs = 92 + ((33 + 4 * n_freq) if (transfer and n_freq) else 0)
     return 4 * rhs + 16 * ni + 3 + 6
 
 
