@@ -706,7 +706,8 @@ far_steps(const SlotView<UNI> &v, const float *hi, float kt)
 }
 
 /* One RK4 step (RK4.cl:37-47) of size hs on the NI integrated reals with
- * the compensated update (value = hi + lo).  With one ray per thread the
+ * the compensated update (value = hi + lo), from the first stage's slopes kk
+ * (overwritten).  With one ray per thread the
  * stage sums, stage states and update run on pairs of components (2j,
  * 2j+1) in packed f32x2, one instruction per pair; an odd last component
  * runs scalar.  The update adds h/6 (k1 + 2 k2 + 2 k3 + k4) to the low part
@@ -715,14 +716,14 @@ far_steps(const SlotView<UNI> &v, const float *hi, float kt)
  * pairs of stage states drop out, measured 6% slower.) */
 template <typename V, int NF>
 __device__ __forceinline__ void
-rk4_packed(const RC<V, NF> &rc, V *hi, V *lo, V hs)
+rk4_packed(const RC<V, NF> &rc, V *hi, V *lo, V hs, V *kk)
 {
 	constexpr int NI = Layout<NF>::NI;
 	constexpr int NP = NI / 2;
 	constexpr bool TAIL = NI & 1;
 	constexpr int LAST = NI - 1;
 	const V hh = bc<V>(0.5f) * hs;
-	V kk[NI], t[NI];
+	V t[NI];
 	float2 H[NP], S2[NP];
 	float tS = 0.0f;
 	const float2 hh2 = make_float2(hh, hh), hs2 = make_float2(hs, hs);
@@ -732,7 +733,6 @@ rk4_packed(const RC<V, NF> &rc, V *hi, V *lo, V hs)
 #pragma unroll
 	for(int j = 0; j < NP; ++j)
 		H[j] = make_float2(hi[PA(j)], hi[PB(j)]);
-	rhs<V, NF>(rc, hi, kk);
 #pragma unroll
 	for(int j = 0; j < NP; ++j) {
 		S2[j] = make_float2(kk[PA(j)], kk[PB(j)]);
@@ -796,6 +796,13 @@ mixed_kernel(const MixedTable T, const __grid_constant__ MixedRender R1,
 	typedef Layout<NF> Y;
 	constexpr int NI = Y::NI;
 	constexpr int L = Lanes<V>::N;
+	/* The first stage does not wait for the step rule: near the hole both run
+	 * side by side.  64^2 rays with 4 frequencies 32.8 -> 31.9 ms, 512 x 384
+	 * near 4.37 -> 4.30, 1024^2 1232 -> 1224.  Its slopes stay in registers
+	 * meanwhile: where the ray's constants do too (more than one render) the
+	 * spills cost 1-2%, more than four frequencies spill as well, and without
+	 * transfer there is little to overlap (333 x 187 rays 24.5 -> 24.9). */
+	constexpr bool EARLY = UNI && NF > 0 && NF <= 4 && L == 1 && !ROLLED;
 	const unsigned FULL = 0xffffffffu;
 	const int lane = threadIdx.x & 31;
 
@@ -804,6 +811,8 @@ mixed_kernel(const MixedTable T, const __grid_constant__ MixedRender R1,
 	Slot S[L];
 	bool exhausted = false;
 	int coast = 0; /* steps until far_steps() is asked again */
+	V k1[NI];      /* a step's first slopes */
+	bool freed = true; /* a slot may wait for a ray (kept where EARLY) */
 	/* accepted steps of this thread; with one slot a 32-bit count, flushed
 	 * at a ray's events (store, dump boundary) once it reaches 2^31: between
 	 * two events a ray takes at most one interval's ticks (< 2^31) */
@@ -831,7 +840,7 @@ mixed_kernel(const MixedTable T, const __grid_constant__ MixedRender R1,
 		 * goes on: an empty thread then asks until the warp ends */
 		if(L > 1)
 			idle |= empty;
-		if(__any_sync(FULL, idle)) {
+		if((!EARLY || freed) && __any_sync(FULL, idle)) {
 #pragma unroll
 			for(int k = 0; k < L; ++k) {
 				bool need = !S[k].active && !exhausted;
@@ -901,6 +910,9 @@ mixed_kernel(const MixedTable T, const __grid_constant__ MixedRender R1,
 				any |= S[k].active;
 			if(!__any_sync(FULL, any))
 				break;
+			/* a ray whose window is empty leaves its slot waiting */
+			if constexpr(EARLY)
+				freed = __any_sync(FULL, !S[0].active && !exhausted);
 		}
 
 		/* step control per slot; finished slots store and free */
@@ -914,14 +926,20 @@ mixed_kernel(const MixedTable T, const __grid_constant__ MixedRender R1,
 				coast = reps > 1 ? 0 : COAST_RETRY;
 			}
 			int cap = s.dh_cap;
+			bool near = false;
 			if(reps == 1) {
 				cap = min(cap, v.n() - s.h);
 				/* the warp decides together: branches taken lane by lane
 				 * cost a third of a lone warp's step */
-				const bool far = is_far<UNI>(v, hi);
-				if(!__all_sync(FULL, far || !s.active)) {
-					const int near = near_ticks<UNI>(v, hi, lo, s.active && !far);
-					cap = far ? cap : near;
+				near = !__all_sync(FULL, is_far<UNI>(v, hi) || !s.active);
+			}
+			if constexpr(EARLY) {
+				const RC<V, NF> sc = step_rc<V, NF, UNI>(rc, R1);
+				if(near) {
+					rhs<V, NF>(sc, hi, k1);
+					const bool far = is_far<UNI>(v, hi);
+					const int dn = near_ticks<UNI>(v, hi, lo, s.active && !far);
+					cap = far ? cap : dn;
 					const bool stop = s.active && cap == 0;
 					if(__any_sync(FULL, stop)) {
 						if(stop) {
@@ -930,9 +948,26 @@ mixed_kernel(const MixedTable T, const __grid_constant__ MixedRender R1,
 							flush_steps<L>(cnt, steps);
 						}
 						__syncwarp();
-						if(!__any_sync(FULL, s.active))
-							continue;
+						freed = true;
+						continue; /* the others ask again: k1 is not kept over this */
 					}
+				} else {
+					rhs<V, NF>(sc, hi, k1);
+				}
+			} else if(near) {
+				const bool far = is_far<UNI>(v, hi);
+				const int dn = near_ticks<UNI>(v, hi, lo, s.active && !far);
+				cap = far ? cap : dn;
+				const bool stop = s.active && cap == 0;
+				if(__any_sync(FULL, stop)) {
+					if(stop) {
+						store_slot<V, NF>(v.render(), s, 0, hi, lo);
+						s.active = false;
+						flush_steps<L>(cnt, steps);
+					}
+					__syncwarp();
+					if(!__any_sync(FULL, s.active))
+						continue;
 				}
 			}
 			dh[0] = s.active ? cap : 0;
@@ -994,9 +1029,20 @@ mixed_kernel(const MixedTable T, const __grid_constant__ MixedRender R1,
 			}
 		} else if constexpr(L == 1) {
 			const RC<V, NF> sc = step_rc<V, NF, UNI>(rc, R1);
+			if constexpr(EARLY) {
+				for(int rep = reps;;) {
+					rk4_packed<V, NF>(sc, hi, lo, hs, k1);
+					if(--rep == 0)
+						break;
+					rhs<V, NF>(sc, hi, k1);
+				}
+			} else {
 #pragma unroll 1
-			for(int rep = 0; rep < reps; ++rep)
-				rk4_packed<V, NF>(sc, hi, lo, hs);
+				for(int rep = 0; rep < reps; ++rep) {
+					rhs<V, NF>(sc, hi, k1);
+					rk4_packed<V, NF>(sc, hi, lo, hs, k1);
+				}
+			}
 		} else {
 			const V hh = bc<V>(0.5f) * hs;
 			V kk[NI], t[NI], sum[NI];
@@ -1038,6 +1084,7 @@ mixed_kernel(const MixedTable T, const __grid_constant__ MixedRender R1,
 		}
 		if(!__any_sync(FULL, ended))
 			continue;
+		freed = true;
 #pragma unroll
 		for(int k = 0; k < L; ++k) {
 			Slot &s = S[k];
