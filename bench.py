@@ -10,7 +10,7 @@ step = one full render (icond + every dump interval of every ray).
 Metric: ray-steps/s = accepted RK4 steps summed over rays / time.
   value       mixed-precision persistent kernel, inputs resident in HBM,
               CUDA events on the launching stream, L2 flushed between steps
-  fp64        the plain FP64 kernel (one launch per dump) on the same render
+  fp64        the plain FP64 kernel on the same render
   e2e         the same metric through the C ABI with host buffers: render
               plus the device-to-host copy of the final state every step
   roofline    FP32 CUDA-core bound (the path has no dense contraction);
