@@ -828,11 +828,12 @@ dyst_mixed_kernel(const MixedTable T, const __grid_constant__ GridParams g, cons
 				double t0 = c->t_init + (double)dump * c->dt_dump;
 				double t1 = c->t_init + (double)(dump + 1) * c->dt_dump;
 				double dt = t1 - t0;
-				dh_step = (int)(dyst_getdt64(dt / (double)c->n_sub) / dt * (double)n);
+				const double ticks = dyst_getdt64(dt / (double)c->n_sub) / dt * (double)n;
+				dh_step = ticks >= 1.0 ? (int)ticks : 0;
 				dtnd = dt / (double)n;
 				dtn = (float)dtnd;
 				h = 0;
-				if(dh_step <= 0) /* zero-length interval: nothing to integrate */
+				if(dh_step == 0) /* zero-length interval: nothing to integrate */
 					h = n;
 				else
 					step = true;

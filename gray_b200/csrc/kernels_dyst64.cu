@@ -383,10 +383,12 @@ dyst_evolve64_kernel(const __grid_constant__ RenderParams p, const __grid_consta
 	}
 	const int n = (int)((INT_MAX / n_sub) * n_sub);
 	const double dts = dt / (double)n_sub;
-	const int dh_step = (int)(dyst_getdt64(dts) / dt * (double)n);
+	/* no steps where the interval's ends round to the same time */
+	const double ticks = dyst_getdt64(dts) / dt * (double)n;
+	const int dh_step = ticks >= 1.0 ? (int)ticks : 0;
 	unsigned cnt = 0;
 	bool quiet = false; /* every ray of the warp stayed in its cell and the box */
-	for(int h = 0; h < n && dh_step != 0;) {
+	for(int h = 0; h < n && dh_step > 0;) {
 		const int dh = dh_step > n - h ? n - h : dh_step;
 		const double hs = ((double)dh * dt) / (double)n, hh = 0.5 * hs;
 		const double h6 = hs / 6.0;

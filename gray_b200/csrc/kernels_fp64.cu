@@ -592,7 +592,9 @@ evolve64_kernel(const __grid_constant__ RenderParams p, double *__restrict__ dat
 				dts = dt / (double)n_sub;
 				idt = 1.0 / dt;
 				plain = !(fabs(dt) > 1e-60 && fabs(dt) < 1e60);
-				cap = (int)(dts / dt * nd);
+				/* no steps where the interval's ends round to the same time */
+				const double c = dts / dt * nd;
+				cap = c >= 1.0 ? (int)c : 0;
 			}
 			/* phys.cl:48-64 getdt() in ticks */
 			const Rad64 R = radius64(p, s[1], s[2], s[3]);

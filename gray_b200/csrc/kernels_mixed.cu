@@ -485,17 +485,27 @@ struct Slot {
 	bool active;
 };
 
-/* Per-dump constants, computed in FP64 exactly like the host loop of
- * sim-org/gray.c:251-252 and driver.cl:93; n is the render's ticks per
- * dump interval. */
-__device__ __forceinline__ void
-start_dump(Slot &S, const MixedRender &c, int n)
+/* Starts the slot's next dump interval, from S.dump on: per-dump constants,
+ * computed in FP64 exactly like the host loop of sim-org/gray.c:251-252 and
+ * driver.cl:93; n is the render's ticks per dump interval.  An interval whose
+ * ends round to the same time (t_init far above dt_dump) has no step count
+ * and leaves the state as it is, as evolving from t to t does; false: no
+ * interval is left before `end`. */
+__device__ __forceinline__ bool
+start_dump(Slot &S, const MixedRender &c, int n, int end)
 {
-	double t      = c.t_init + (double)S.dump * c.dt_dump;
-	double target = c.t_init + (double)(S.dump + 1) * c.dt_dump;
-	double dt     = target - t;
-	double dts    = dt / (double)c.n_sub;
-	S.dh_cap = (int)(dts / dt * (double)n);
+	double dt = 0.0;
+	for(; S.dump < end; ++S.dump) {
+		double t      = c.t_init + (double)S.dump * c.dt_dump;
+		double target = c.t_init + (double)(S.dump + 1) * c.dt_dump;
+		dt = target - t;
+		if(fabs(dt) > 0.0)
+			break;
+	}
+	if(S.dump >= end)
+		return false;
+	const double dts = dt / (double)c.n_sub, cap = dts / dt * (double)n;
+	S.dh_cap = cap >= 1.0 ? (int)cap : 0; /* an infinite interval has none either */
 	S.cdt    = (float)((double)n / fabs(dt));
 	S.dtn    = (float)(dt / (double)n);
 	S.h      = 0;
@@ -505,6 +515,7 @@ start_dump(Slot &S, const MixedRender &c, int n)
 	const double e_cap = sqrt((double)S.dh_cap / (0.01 * (double)S.cdt));
 	const double r_far = 1.01 * ((double)c.rp_d + e_cap) + 1.0;
 	S.r2_far = (float)(r_far * r_far);
+	return true;
 }
 
 /* A slot's render-wide values: from the slot (loaded with the ray) or, with
@@ -879,7 +890,7 @@ mixed_kernel(const MixedTable T, const __grid_constant__ MixedRender R1,
 #pragma unroll
 				for(int i = 0; i < 8; ++i)
 					s0[i] = c.data[i * nr + s.ray];
-				if(s.dump >= c.dump_end) { /* empty window: state unchanged */
+				if(!start_dump(s, c, c.n_ticks, c.dump_end)) { /* empty window: state unchanged */
 					c.info[s.ray] = getuu_d(c.a_d, s0);
 					continue;
 				}
@@ -901,7 +912,6 @@ mixed_kernel(const MixedTable T, const __grid_constant__ MixedRender R1,
 					setl(hi[i], k, h);
 					setl(lo[i], k, (float)(v[i] - (double)h));
 				}
-				start_dump(s, c, c.n_ticks);
 				s.active = true;
 			}
 			bool any = false;
@@ -1091,11 +1101,10 @@ mixed_kernel(const MixedTable T, const __grid_constant__ MixedRender R1,
 			const SlotView<UNI> v{s, R1};
 			if(s.active && s.h >= v.n()) {
 				flush_steps<L>(cnt, steps);
-				if(++s.dump >= v.dump_end()) {
+				++s.dump;
+				if(!start_dump(s, v.render(), v.n(), v.dump_end())) {
 					store_slot<V, NF>(v.render(), s, k, hi, lo);
 					s.active = false;
-				} else {
-					start_dump(s, v.render(), v.n());
 				}
 			}
 		}
