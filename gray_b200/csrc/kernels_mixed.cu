@@ -485,25 +485,34 @@ struct Slot {
 	bool active;
 };
 
-/* Starts the slot's next dump interval, from S.dump on: per-dump constants,
- * computed in FP64 exactly like the host loop of sim-org/gray.c:251-252 and
- * driver.cl:93; n is the render's ticks per dump interval.  An interval whose
- * ends round to the same time (t_init far above dt_dump) has no step count
- * and leaves the state as it is, as evolving from t to t does; false: no
- * interval is left before `end`. */
-__device__ __forceinline__ bool
-start_dump(Slot &S, const MixedRender &c, int n, int end)
+/* The length of a dump interval as the host loop of sim-org/gray.c:251-252
+ * computes it. */
+__device__ __forceinline__ double
+dump_length(const MixedRender &c, int dump)
 {
-	double dt = 0.0;
-	for(; S.dump < end; ++S.dump) {
-		double t      = c.t_init + (double)S.dump * c.dt_dump;
-		double target = c.t_init + (double)(S.dump + 1) * c.dt_dump;
-		dt = target - t;
-		if(fabs(dt) > 0.0)
-			break;
-	}
-	if(S.dump >= end)
-		return false;
+	const double t      = c.t_init + (double)dump * c.dt_dump;
+	const double target = c.t_init + (double)(dump + 1) * c.dt_dump;
+	return target - t;
+}
+
+/* The first dump interval from `dump` on that has a length.  One whose ends
+ * round to the same time (t_init far above dt_dump) has no step count and
+ * leaves the state as it is, as evolving from t to t does.  Out of line, and
+ * asked once per interval: inlined it cost the stepping loop 1-2% in spills. */
+__device__ __noinline__ int
+next_dump(const MixedRender &c, int dump)
+{
+	while(dump < c.dump_end && !(fabs(dump_length(c, dump)) > 0.0))
+		++dump;
+	return dump;
+}
+
+/* Per-dump constants, computed in FP64 exactly like driver.cl:93; n is the
+ * render's ticks per dump interval. */
+__device__ __forceinline__ void
+start_dump(Slot &S, const MixedRender &c, int n)
+{
+	const double dt  = dump_length(c, S.dump);
 	const double dts = dt / (double)c.n_sub, cap = dts / dt * (double)n;
 	S.dh_cap = cap >= 1.0 ? (int)cap : 0; /* an infinite interval has none either */
 	S.cdt    = (float)((double)n / fabs(dt));
@@ -515,7 +524,6 @@ start_dump(Slot &S, const MixedRender &c, int n, int end)
 	const double e_cap = sqrt((double)S.dh_cap / (0.01 * (double)S.cdt));
 	const double r_far = 1.01 * ((double)c.rp_d + e_cap) + 1.0;
 	S.r2_far = (float)(r_far * r_far);
-	return true;
 }
 
 /* A slot's render-wide values: from the slot (loaded with the ray) or, with
@@ -874,7 +882,7 @@ mixed_kernel(const MixedTable T, const __grid_constant__ MixedRender R1,
 				const MixedRender &c = UNI ? R1 : T.renders[rdx];
 				Slot &s = S[k];
 				s.ray = (unsigned int)(UNI ? g : g - T.prefix[rdx]);
-				s.dump = c.dump_begin;
+				s.dump = next_dump(c, c.dump_begin);
 				if constexpr(!UNI) {
 					s.c = &c;
 					s.n = c.n_ticks;
@@ -890,7 +898,7 @@ mixed_kernel(const MixedTable T, const __grid_constant__ MixedRender R1,
 #pragma unroll
 				for(int i = 0; i < 8; ++i)
 					s0[i] = c.data[i * nr + s.ray];
-				if(!start_dump(s, c, c.n_ticks, c.dump_end)) { /* empty window: state unchanged */
+				if(s.dump >= c.dump_end) { /* empty window: state unchanged */
 					c.info[s.ray] = getuu_d(c.a_d, s0);
 					continue;
 				}
@@ -912,6 +920,7 @@ mixed_kernel(const MixedTable T, const __grid_constant__ MixedRender R1,
 					setl(hi[i], k, h);
 					setl(lo[i], k, (float)(v[i] - (double)h));
 				}
+				start_dump(s, c, c.n_ticks);
 				s.active = true;
 			}
 			bool any = false;
@@ -920,7 +929,6 @@ mixed_kernel(const MixedTable T, const __grid_constant__ MixedRender R1,
 				any |= S[k].active;
 			if(!__any_sync(FULL, any))
 				break;
-			/* a ray whose window is empty leaves its slot waiting */
 			if constexpr(EARLY)
 				freed = __any_sync(FULL, !S[0].active && !exhausted);
 		}
@@ -1101,10 +1109,12 @@ mixed_kernel(const MixedTable T, const __grid_constant__ MixedRender R1,
 			const SlotView<UNI> v{s, R1};
 			if(s.active && s.h >= v.n()) {
 				flush_steps<L>(cnt, steps);
-				++s.dump;
-				if(!start_dump(s, v.render(), v.n(), v.dump_end())) {
+				s.dump = next_dump(v.render(), s.dump + 1);
+				if(s.dump >= v.dump_end()) {
 					store_slot<V, NF>(v.render(), s, k, hi, lo);
 					s.active = false;
+				} else {
+					start_dump(s, v.render(), v.n());
 				}
 			}
 		}
