@@ -923,7 +923,9 @@ mixed_kernel(const MixedTable T, const __grid_constant__ MixedRender R1,
 				start_dump(s, c, c.n_ticks);
 				s.active = true;
 			}
-			bool any = false;
+			/* a ray whose window is empty leaves its slot waiting, and a warp
+			 * that drew nothing else asks again until the queue is out */
+			bool any = !exhausted;
 #pragma unroll
 			for(int k = 0; k < L; ++k)
 				any |= S[k].active;
