@@ -623,9 +623,10 @@ flat_steps(const GridParams &g, int m, bool step, int &h, int n, int dh_step,
 	float far = d > 0.0f ? fminf(0.99f * d * rcp_a(dx + 1e-30f), 1e6f) - 2.0f : 0.0f;
 	far = fmaxf(far, __shfl_xor_sync(FULL, far, 1));
 	far = fmaxf(far, __shfl_xor_sync(FULL, far, 2));
-	/* u's own update must be a fixed point */
+	/* u's own update must be a fixed point, and x may not overflow on the way
+	 * (a ray whose state does, or is not finite, ends at that step) */
 	const float tu = uh - ul;
-	const bool still = tu == uh && (tu - uh) + ul == ul;
+	const bool still = tu == uh && (tu - uh) + ul == ul && fabsf(xh) <= 1e30f && dx <= 1e24f;
 	int todo = far >= 1.0f ? (int)far : 0;
 	const int left = step ? (n - h - 1) / dh_step : INT_MAX; /* not the last step */
 	todo = !step ? INT_MAX : still ? min(todo, left) : 0;
