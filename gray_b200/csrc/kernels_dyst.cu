@@ -331,13 +331,17 @@ struct Axis {
 	int tag;           /* the cell index (lane 0: level code) in Cell    */
 };
 
-/* the levels in use: bit 0 level 0, bit 1 level 1; a level of weight zero
- * (t outside [t1, t2] in physics mode, where the factor is clamped) is not
- * read */
+/* the levels in use: bit 0 level 0, bit 1 level 1.  In physics mode the time
+ * factor is clamped to [0, 1] and a level of weight zero is not read; in
+ * reference semantics, which two levels always run with LV = 2, the fields
+ * extrapolate (interp.cl:183-205): both at any time, none at a NaN */
+template <int LV>
 __device__ __forceinline__ int
-level_code(bool single, float ft)
+level_code(const GridParams &g, float ft)
 {
-	return single ? 1 : (ft < 1.0f ? 1 : 0) | (ft > 0.0f ? 2 : 0);
+	if(LV == 2 && !g.physics)
+		return ft == ft ? 3 : 0;
+	return g.single ? 1 : (ft < 1.0f ? 1 : 0) | (ft > 0.0f ? 2 : 0);
 }
 
 template <bool RT>
@@ -437,11 +441,15 @@ enter_cell(const GridParams &g, const DystConst &dc, Axis &A, Cell<RT> &C, int l
 				if(g.physics)
 					w = fminf(fmaxf(w, 0.0f), 1.0f);
 			}
-			i0 = level_code(g.single, w);
+			i0 = level_code<LV>(g, w);
 			/* times at which the rounded factor surely gives the same code */
 			const float mg = 1e-5f * (fabsf(lo) + fabsf(hi));
 			A.xa = i0 == 2 ? hi + mg : i0 == 3 ? lo + mg : -INFINITY;
 			A.xb = i0 == 1 ? (g.single ? INFINITY : lo) : i0 == 3 ? hi - mg : INFINITY;
+			if(LV == 2 && !g.physics) {
+				A.xa = -INFINITY;
+				A.xb = INFINITY;
+			}
 			if(i0 == 0 || (LV == 1 && i0 == 3))
 				A.xa = INFINITY;
 		} else {
