@@ -9,13 +9,16 @@
  * sit exactly where the oracle (oracle/gray_oracle.c) places its fma()
  * calls.  FP64 '/' and sqrt() are IEEE round-to-nearest on sm_100, as in
  * the oracle, so the geodesic agrees bit for bit; the stepping loop's own
- * quotients and roots (below) round the same.
+ * quotients and roots (round64.cuh) round the same.
  */
 #include <climits>
 
 #include "gray_internal.h"
+#include "round64.cuh"
 
 namespace {
+
+using namespace round64;
 
 constexpr int EVOLVE64_BLOCK = 64;
 
@@ -28,98 +31,12 @@ getrr64(const RenderParams &p, double x, double y, double z)
 	return sqrt(fma(kk, kk, p.aa * zz)) + kk;
 }
 
-/* ------------------------- correctly rounded quotients and square roots */
-
-/* The stepping loop takes five quotients and two roots per RHS.  The
- * operators cost a range check and a branch each, which also keeps the
- * independent ones from overlapping: a lone warp spent 2.3 us per step.
- * These are the fused multiply-add iterations of Markstein (IBM J. Res. Dev.
- * 34, 1990; "IA-64 and Elementary Functions", 2000): Newton-Raphson or
- * Goldschmidt steps from a hardware seed, then a correction by the exact
- * residual, which rounds to nearest.  (Against the operators on 5e9 random
- * operands each they differ, by one ulp, only where a divisor's significand
- * is all ones, Markstein's known exception.)  They hold for operands far
- * from the ends of the exponent range; one check per RHS (in_range) sends
- * everything else, zeros, infinities and NaN to the operators. */
-__device__ __forceinline__ double
-seed_rcp(double b)
-{
-	double y;
-	asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-	return y;
-}
-
-__device__ __forceinline__ double
-seed_rsqrt(double x)
-{
-	double y;
-	asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-	return y;
-}
-
-/* 1/b from y within a few ulp of it */
-__device__ __forceinline__ double
-rcp_near(double b, double y)
-{
-	return fma(y, fma(-b, y, 1.0), y);
-}
-
-/* 1/b to within an ulp or so, from y within 2^-18 of it */
-__device__ __forceinline__ double
-rcp_from(double b, double y)
-{
-	const double e = fma(-b, y, 1.0);
-	return fma(y, fma(e, e, e), y); /* cubic */
-}
-
-__device__ __forceinline__ double
-rcp_fast(double b)
-{
-	return rcp_from(b, seed_rcp(b));
-}
-
-/* 1/b */
-__device__ __forceinline__ double
-rcp_rn(double b)
-{
-	return rcp_near(b, rcp_fast(b));
-}
-
-/* a/b with y = 1/b rounded to nearest */
-__device__ __forceinline__ double
-div_rn(double a, double b, double y)
-{
-	const double q = a * y;
-	return fma(fma(-b, q, a), y, q);
-}
-
-/* sqrt(x), and h = 1/(2 sqrt(x)) to within an ulp or so, from y0 within 2^-18
- * of 1/sqrt(x): one cubic step, e^3 < 2^-50 of which a 5/16th is left out */
-__device__ __forceinline__ double
-sqrt_from(double x, double y0, double &h)
-{
-	const double g0 = x * y0, h0 = 0.5 * y0;
-	const double e = fma(-g0, y0, 1.0), c = fma(0.375, e, 0.5);
-	const double g = fma(g0 * e, c, g0);
-	h = fma(h0 * e, c, h0);
-	return fma(fma(-g, g, x), h, g);
-}
-
-/* sqrt(x), and y = 1/sqrt(x) to within an ulp or so */
-__device__ __forceinline__ double
-sqrt_rn(double x, double &y)
-{
-	double h;
-	const double r = sqrt_from(x, seed_rsqrt(x), h);
-	y = h + h;
-	return r;
-}
-
 /* The radius at an event (KS.cl:48-55, 289-295): what the step rule and the
  * first RHS of a step share.  Valid where in_range(). */
 struct Rad64 {
 	double zz, dd, rr, r;
 	double hd, yr, yq; /* about 1/(2 dd), 1/r; within 2^-18 of 1/rr */
+	bool ones;         /* all_ones() of a radicand           */
 };
 
 /* where every operand of the loop's quotients and roots is normal with room
@@ -129,7 +46,7 @@ struct Rad64 {
 __device__ __forceinline__ bool
 in_range(const Rad64 &R)
 {
-	return R.rr > 1e-6 && R.rr < 1e60 && R.rr >= R.dd;
+	return R.rr > 1e-6 && R.rr < 1e60 && R.rr >= R.dd && !R.ones;
 }
 
 /* A lone warp's step is one chain of dependent operations, and the seeds of
@@ -153,11 +70,13 @@ radius64(const RenderParams &p, double x, double y, double z)
 	double hr;
 	R.r = sqrt_from(R.rr, yr, hr);
 	R.yr = hr + hr;
+	R.ones = all_ones(d2) | all_ones(R.rr);
 	return R;
 }
 
 struct Aux64 {
 	double r, f, lx, ly, lz, flu, iss, ir;
+	bool ones; /* all_ones() of a divisor */
 };
 
 /* KS.cl:263-378 gr_rhs(), Chan et al. form; returns f, l and f l.u for the
@@ -185,6 +104,7 @@ ks_rhs64(const RenderParams &p, const Rad64 &R, const double *s, double *ds, Aux
 			iss = 1.0 / ss;
 			hrd = 0.5 / rd;
 			t2  = 2.0 / (rr + az / rr);
+			aux.ones = false;
 		} else {
 			/* a power of 2 over b is that power of 1/b, exactly; 1/rr from
 			 * its own seed, so that it does not wait for the root; and
@@ -194,6 +114,7 @@ ks_rhs64(const RenderParams &p, const Rad64 &R, const double *s, double *ds, Aux
 			hrd = 0.5 * rcp_near(rd, rcp_near(rd, R.yr * (R.hd + R.hd)));
 			const double den = rr + div_rn(az, rr, rcp_near(rr, rcp_from(rr, R.yq)));
 			t2  = 2.0 * rcp_near(den, rcp_near(den, R.hd));
+			aux.ones = all_ones(ss) | all_ones(rd) | all_ones(den);
 		}
 		tmp  = hrd;
 		dz_r = (tmp * ss) * z;
@@ -387,35 +308,51 @@ rhs_any64(const RenderParams &p, const double *s, double *ds)
 	R.rr = R.dd + kk;
 	R.r = sqrt(R.rr);
 	R.hd = R.yr = R.yq = 0.0;
+	R.ones = false;
 	ks_rhs64<true>(p, R, s, ds, aux);
 	if constexpr(NF > 0)
 		torus_any64<NF>(p, s, aux, ds + 8);
 }
 
-/* phys.cl:66-74 rhs() */
+/* RK4.cl:37-47 integrate() by dt, h6 = dt / 6, with the operators */
 template <int NF>
-__device__ __forceinline__ void
+__device__ __noinline__ void
+rk4_any64(const RenderParams &p, double *s, double dt, double h6)
+{
+	constexpr int ND = 8 + 2 * NF;
+	double k1[ND], k2[ND], k[ND], t[ND];
+	const double hdt = 0.5 * dt;
+	rhs_any64<NF>(p, s, k1);
+	for(int i = 0; i < ND; ++i) t[i] = fma(hdt, k1[i], s[i]);
+	rhs_any64<NF>(p, t, k2);
+	for(int i = 0; i < ND; ++i) t[i] = fma(hdt, k2[i], s[i]);
+	rhs_any64<NF>(p, t, k);
+	for(int i = 0; i < ND; ++i) {
+		t[i] = fma(dt, k[i], s[i]);
+		k2[i] = k2[i] + k[i];
+	}
+	rhs_any64<NF>(p, t, k);
+	for(int i = 0; i < ND; ++i)
+		s[i] = fma(h6, fma(2.0, k2[i], k1[i]) + k[i], s[i]);
+}
+
+/* phys.cl:66-74 rhs(); false: operands that the loop's own quotients and
+ * roots do not hold for */
+template <int NF>
+__device__ __forceinline__ bool
 rhs64(const RenderParams &p, const Torus64 &T, const Rad64 &R, const double *s, double *ds)
 {
 	Aux64 aux;
-	bool ok = in_range(R);
+	bool ok = in_range(R) && !all_ones(R.r);
 	ks_rhs64<false>(p, R, s, ds, aux);
 	if constexpr(NF > 0)
 		ok = torus_rt64<NF>(p, T, ok, s, aux, ds);
-	if(!ok) {
-		/* copies: what a call is given by address lives in memory */
-		double sc[8 + 2 * NF], any[8 + 2 * NF];
-#pragma unroll
-		for(int i = 0; i < 8 + 2 * NF; ++i)
-			sc[i] = s[i];
-		rhs_any64<NF>(p, sc, any);
-#pragma unroll
-		for(int i = 0; i < 8 + 2 * NF; ++i)
-			ds[i] = any[i];
-	}
+	return ok && !aux.ones;
 }
 
-/* RK4.cl:37-47 integrate() by dt, h6 = dt / 6; R: the radius at s */
+/* RK4.cl:37-47 integrate() by dt, h6 = dt / 6; R: the radius at s.  A step
+ * that met such operands is taken again with the operators: asked once per
+ * step, the question does not stand between the stages. */
 template <int NF>
 __device__ __forceinline__ void
 rk4_64(const RenderParams &p, const Torus64 &T, const Rad64 &R, double *s, double dt, double h6)
@@ -423,22 +360,34 @@ rk4_64(const RenderParams &p, const Torus64 &T, const Rad64 &R, double *s, doubl
 	constexpr int ND = 8 + 2 * NF;
 	double k1[ND], k2[ND], k[ND], t[ND];
 	const double hdt = 0.5 * dt;
-	rhs64<NF>(p, T, R, s, k1);
+	bool ok = rhs64<NF>(p, T, R, s, k1);
 #pragma unroll
 	for(int i = 0; i < ND; ++i) t[i] = fma(hdt, k1[i], s[i]);
-	rhs64<NF>(p, T, radius64(p, t[1], t[2], t[3]), t, k2);
+	ok &= rhs64<NF>(p, T, radius64(p, t[1], t[2], t[3]), t, k2);
 #pragma unroll
 	for(int i = 0; i < ND; ++i) t[i] = fma(hdt, k2[i], s[i]);
-	rhs64<NF>(p, T, radius64(p, t[1], t[2], t[3]), t, k);
+	ok &= rhs64<NF>(p, T, radius64(p, t[1], t[2], t[3]), t, k);
 #pragma unroll
 	for(int i = 0; i < ND; ++i) {
 		t[i] = fma(dt, k[i], s[i]);
 		k2[i] = k2[i] + k[i]; /* k2 + k3 */
 	}
-	rhs64<NF>(p, T, radius64(p, t[1], t[2], t[3]), t, k);
+	ok &= rhs64<NF>(p, T, radius64(p, t[1], t[2], t[3]), t, k);
+	if(ok) {
 #pragma unroll
-	for(int i = 0; i < ND; ++i)
-		s[i] = fma(h6, fma(2.0, k2[i], k1[i]) + k[i], s[i]);
+		for(int i = 0; i < ND; ++i)
+			s[i] = fma(h6, fma(2.0, k2[i], k1[i]) + k[i], s[i]);
+	} else {
+		/* a copy: what a call is given by address lives in memory */
+		double any[ND];
+#pragma unroll
+		for(int i = 0; i < ND; ++i)
+			any[i] = s[i];
+		rk4_any64<NF>(p, any, dt, h6);
+#pragma unroll
+		for(int i = 0; i < ND; ++i)
+			s[i] = any[i];
+	}
 }
 
 /* f and l_mu at q with the operation sequence of ks_rhs64() */

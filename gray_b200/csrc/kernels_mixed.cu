@@ -39,6 +39,7 @@
 #include "gray_internal.h"
 #include "logk2_table.h"
 #include "mixed_table.h"
+#include "round64.cuh"
 
 namespace {
 
@@ -379,41 +380,22 @@ rhs(const RC<V, NF> &c, const V *s, V *ds)
 
 /* ---------------------------------------------------------- FP64 islands */
 
-/* sqrt(x) rounded to nearest, for x far from the ends of the exponent range,
- * from y0 within 2^-18 of 1/sqrt(x): a cubic step, then Markstein's
- * correction by the exact residual ("IA-64 and Elementary Functions", 2000).
- * The step rule near the horizon waits for two roots, and 10^4 steps run
- * there; the operator's range check and branch keep them from overlapping
- * with anything. */
-__device__ __forceinline__ double
-sqrt_rn_d(double x, double y0)
-{
-	const double g0 = x * y0, h0 = 0.5 * y0;
-	const double e = fma(-g0, y0, 1.0), c = fma(0.375, e, 0.5);
-	const double g = fma(g0 * e, c, g0), h = fma(h0 * e, c, h0);
-	return fma(fma(-g, g, x), h, g);
-}
-
-__device__ __forceinline__ double
-rsqrt_seed(double x)
-{
-	double y;
-	asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-	return y;
-}
-
-/* KS.cl:48-55 radius; the second root's seed comes from r^2 to 2^-19, known
- * before the first is refined.  Where r^2 cancels or is far out of range by
- * the operators, if the answer is wanted (on). */
+/* KS.cl:48-55 radius, for the step rule near the horizon: it waits for two
+ * roots, and 10^4 steps run there, so they are round64.cuh's.  The second
+ * root's seed comes from r^2 to 2^-19, known before the first is refined.
+ * Where r^2 cancels or is far out of range by the operators, if the answer is
+ * wanted (on).  (An ulp of a radicand of all ones does not reach the FP32
+ * result.) */
 __device__ __forceinline__ double
 getr_d(double aa, double x, double y, double z, bool on)
 {
 	const double zz = z * z;
 	const double kk = 0.5 * (fma(x, x, fma(y, y, zz)) - aa);
-	const double d2 = fma(kk, kk, aa * zz), y0 = rsqrt_seed(d2);
-	const double y1 = rsqrt_seed(fma(d2, y0, kk));
-	const double dd = sqrt_rn_d(d2, y0), rr = dd + kk;
-	double r = sqrt_rn_d(rr, y1);
+	const double d2 = fma(kk, kk, aa * zz), y0 = round64::seed_rsqrt(d2);
+	const double y1 = round64::seed_rsqrt(fma(d2, y0, kk));
+	double h;
+	const double dd = round64::sqrt_from(d2, y0, h), rr = dd + kk;
+	double r = round64::sqrt_from(rr, y1, h);
 	if(on && !(rr > 1e-6 && rr < 1e60 && rr >= dd))
 		r = sqrt(sqrt(d2) + kk);
 	return r;
