@@ -158,6 +158,15 @@ make_params(const gray_render_desc *d, RenderParams *p)
 	p->torus_n0 = d->torus_n0;
 	p->torus_kappa = d->torus_kappa;
 	p->torus_hr = d->torus_hr;
+	{
+		const double q = sqrt(p->rp), ql = fma(-q, q, p->rp) / (2.0 * q);
+		const double t = p->torus_n0 * p->rp, tl = fma(p->torus_n0, p->rp, -t);
+		p->torus_n15  = t * q;
+		p->torus_n15l = fma(t, q, -p->torus_n15) + (t * ql + tl * q);
+		const double h2 = p->torus_hr * p->torus_hr, h2l = fma(p->torus_hr, p->torus_hr, -h2);
+		p->torus_ig  = 0.5 / h2;
+		p->torus_igl = (fma(-2.0 * p->torus_ig, h2, 1.0) - 2.0 * p->torus_ig * h2l) * p->torus_ig;
+	}
 	for(int i = 0; i < d->n_freq; ++i) {
 		p->nupow[i]  = pow(d->nu[i], -0.7);
 		p->nuinv2[i] = 1.0 / (d->nu[i] * d->nu[i]);

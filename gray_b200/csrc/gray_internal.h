@@ -41,6 +41,8 @@ struct RenderParams {
 	long long row0;          /* first camera row of the render's rays    */
 	int    n_freq, flow, n_data, spacetime;
 	double torus_n0, torus_kappa, torus_hr;
+	/* n0 r_+^1.5 and 1 / (2 h_r^2) with their rounding (FP64 transfer) */
+	double torus_n15, torus_n15l, torus_ig, torus_igl;
 	double nupow[GRAY_MAX_FREQ];   /* nu_i^-0.7 */
 	double nuinv2[GRAY_MAX_FREQ];  /* nu_i^-2   */
 	float  nupow_f[GRAY_MAX_FREQ];

@@ -237,22 +237,18 @@ torus_any64(const RenderParams &p, const double *s, const Aux64 &x, double *ds)
 	}
 }
 
-/* The torus's render-wide factors */
-struct Torus64 {
-	double n0rp15; /* n0 r_+^1.5      */
-	double ihr2;   /* 1 / (2 h_r^2)   */
-};
-
-/* The same transfer with 1/r and its root shared (the density is n0 r_+^1.5
- * r^-1.5 e^-g, g = (z/r)^2 / (2 h_r^2)) and one exponential per frequency for
- * e^-g shift^-0.7 e^-tau_i; every step is good to about an ulp.  Returns
- * whether its operands were in the ranges this holds in, given ok of the RHS.  (With pow,
- * the Gaussian and e^-tau_i apart and seven more quotients, transfer took
- * three quarters of a step's time at four frequencies.) */
+/* The same transfer with 1/r and its root shared: the density is n0 r_+^1.5
+ * r^-1.5 e^-g, g = (z/r)^2 / (2 h_r^2).  What the shared factors add to the
+ * rounding is carried along where it costs an operation or two (z/r rounded
+ * to nearest, r^-1.5 and the render's constants with their low parts), so that
+ * the mean error is not above that of the operators, pow and exp; one
+ * exponential per frequency of the three exponents' sum had up to 1.3 times
+ * theirs, as its error grows with its argument.  Returns whether its operands
+ * were in the ranges this holds in, given ok of the RHS.  (With the operators,
+ * transfer took three quarters of a step's time at four frequencies.) */
 template <int NF>
 __device__ __forceinline__ bool
-torus_rt64(const RenderParams &p, const Torus64 &T, bool ok, const double *s, const Aux64 &x,
-           double *ds)
+torus_rt64(const RenderParams &p, bool ok, const double *s, const Aux64 &x, double *ds)
 {
 	bool emits = false;
 	double shift = 1.0, irs = 0.0;
@@ -273,23 +269,26 @@ torus_rt64(const RenderParams &p, const Torus64 &T, bool ok, const double *s, co
 		emits = D > 0.0 && !(shift <= 0.0);
 		ok = ok && (!emits || (D > 1e-30 && shift > 1e-9 && shift < 1e9));
 	}
+	double n = 0.0;
+	if(emits) {
+		const double v = div_rn(s[3], x.r, x.ir), v2 = v * v;
+		const double w = x.ir * irs, wl = fma(x.ir, irs, -w);
+		const double g = fma(v2, p.torus_ig, v2 * p.torus_igl);
+		n = fma(w, p.torus_n15, fma(w, p.torus_n15l, wl * p.torus_n15)) * exp(-g);
+		emits = n != 0.0;
+	}
 	if(!emits || !ok) {
 #pragma unroll
 		for(int i = 0; i < 2 * NF; ++i)
 			ds[8 + i] = 0.0;
 		return ok;
 	}
-	const double g = (x.lz * x.lz) * T.ihr2;
-	const double n15 = T.n0rp15 * (x.ir * irs);
-	const double n = n15 * exp(-g);
-	const double ish  = rcp_fast(shift);
-	const double tfac = (p.torus_kappa * n) * ish;
+	const double tfac = (p.torus_kappa * n) * rcp_fast(shift);
 	const double is2  = rcp_fast(fma(shift, shift, GRAY_EPSILON));
-	const double jfac = n15 * is2;
-	const double arg  = fma(-0.7, log(shift), -g);
+	const double jfac = (n * is2) * pow_m07(shift);
 #pragma unroll
 	for(int i = 0; i < NF; ++i) {
-		ds[8 + i]      = -((jfac * p.nupow[i]) * exp(arg - s[8 + NF + i]));
+		ds[8 + i]      = -((jfac * p.nupow[i]) * exp(-s[8 + NF + i]));
 		ds[8 + NF + i] = -(tfac * p.nuinv2[i]);
 	}
 	return true;
@@ -340,13 +339,13 @@ rk4_any64(const RenderParams &p, double *s, double dt, double h6)
  * roots do not hold for */
 template <int NF>
 __device__ __forceinline__ bool
-rhs64(const RenderParams &p, const Torus64 &T, const Rad64 &R, const double *s, double *ds)
+rhs64(const RenderParams &p, const Rad64 &R, const double *s, double *ds)
 {
 	Aux64 aux;
 	bool ok = in_range(R) && !all_ones(R.r);
 	ks_rhs64<false>(p, R, s, ds, aux);
 	if constexpr(NF > 0)
-		ok = torus_rt64<NF>(p, T, ok, s, aux, ds);
+		ok = torus_rt64<NF>(p, ok, s, aux, ds);
 	return ok && !aux.ones;
 }
 
@@ -355,24 +354,24 @@ rhs64(const RenderParams &p, const Torus64 &T, const Rad64 &R, const double *s, 
  * step, the question does not stand between the stages. */
 template <int NF>
 __device__ __forceinline__ void
-rk4_64(const RenderParams &p, const Torus64 &T, const Rad64 &R, double *s, double dt, double h6)
+rk4_64(const RenderParams &p, const Rad64 &R, double *s, double dt, double h6)
 {
 	constexpr int ND = 8 + 2 * NF;
 	double k1[ND], k2[ND], k[ND], t[ND];
 	const double hdt = 0.5 * dt;
-	bool ok = rhs64<NF>(p, T, R, s, k1);
+	bool ok = rhs64<NF>(p, R, s, k1);
 #pragma unroll
 	for(int i = 0; i < ND; ++i) t[i] = fma(hdt, k1[i], s[i]);
-	ok &= rhs64<NF>(p, T, radius64(p, t[1], t[2], t[3]), t, k2);
+	ok &= rhs64<NF>(p, radius64(p, t[1], t[2], t[3]), t, k2);
 #pragma unroll
 	for(int i = 0; i < ND; ++i) t[i] = fma(hdt, k2[i], s[i]);
-	ok &= rhs64<NF>(p, T, radius64(p, t[1], t[2], t[3]), t, k);
+	ok &= rhs64<NF>(p, radius64(p, t[1], t[2], t[3]), t, k);
 #pragma unroll
 	for(int i = 0; i < ND; ++i) {
 		t[i] = fma(dt, k[i], s[i]);
 		k2[i] = k2[i] + k[i]; /* k2 + k3 */
 	}
-	ok &= rhs64<NF>(p, T, radius64(p, t[1], t[2], t[3]), t, k);
+	ok &= rhs64<NF>(p, radius64(p, t[1], t[2], t[3]), t, k);
 	if(ok) {
 #pragma unroll
 		for(int i = 0; i < ND; ++i)
@@ -520,9 +519,6 @@ evolve64_kernel(const __grid_constant__ RenderParams p, double *__restrict__ dat
 		for(int c = 0; c < ND; ++c)
 			s[c] = data[c * nr + g];
 
-		Torus64 T;
-		T.n0rp15 = (p.torus_n0 * p.rp) * sqrt(p.rp);
-		T.ihr2 = 0.5 / (p.torus_hr * p.torus_hr);
 		const int n = (int)((INT_MAX / n_sub) * n_sub);
 		const double nd = (double)n, in = 1.0 / nd, i6 = 1.0 / 6.0;
 		double dt = 0.0, dts = 0.0, idt = 0.0;
@@ -561,7 +557,7 @@ evolve64_kernel(const __grid_constant__ RenderParams p, double *__restrict__ dat
 				dh = n - h;
 			const double a = (double)dh * dt;
 			const double hs = plain ? a / nd : div_rn(a, nd, in);
-			rk4_64<NF>(p, T, R, s, hs, plain ? hs / 6.0 : div_rn(hs, 6.0, i6));
+			rk4_64<NF>(p, R, s, hs, plain ? hs / 6.0 : div_rn(hs, 6.0, i6));
 			h += dh;
 			++cnt;
 		}

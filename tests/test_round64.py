@@ -37,6 +37,23 @@ __global__ void check(const double *x, const double *a, long long n, unsigned lo
 		atomicAdd(bad + 2, (unsigned long long)(rcp_near(b, rcp_near(b, fma(r, k * 0x1p-52, r))) != r));
 	atomicAdd(bad + 3, (unsigned long long)(div_rn(a[i], b, r) != a[i] / b));
 }
+__global__ void powers(const double *x, double *y, long long n)
+{
+	const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+	if(i < n)
+		y[i] = pow_m07(x[i]);
+}
+extern "C" int pow_run(const double *x, double *y, long long n)
+{
+	double *d = 0;
+	if(cudaMalloc(&d, 2 * n * sizeof(double)))
+		return 1;
+	cudaMemcpy(d, x, n * sizeof(double), cudaMemcpyHostToDevice);
+	powers<<<(unsigned)((n + 255) / 256), 256>>>(d, d + n, n);
+	cudaError_t e = cudaMemcpy(y, d + n, n * sizeof(double), cudaMemcpyDeviceToHost);
+	cudaFree(d);
+	return e != cudaSuccess;
+}
 extern "C" int run(const double *x, const double *a, long long n, unsigned long long *out)
 {
 	double *d = 0;
@@ -102,18 +119,40 @@ def test_the_hard_radicands_are_hard():
         assert min(abs(v - q * q) for q in (t - 2, t, t + 2)) < 256
 
 
-@pytest.mark.gpu
-def test_equal_to_the_operators(tmp_path):
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
     if not os.path.exists(NVCC):
         pytest.skip("no nvcc")
-    src, lib = tmp_path / "r.cu", tmp_path / "libr.so"
-    src.write_text(SRC)
+    d = tmp_path_factory.mktemp("round64")
+    (d / "r.cu").write_text(SRC)
     subprocess.check_call([NVCC, "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-fmad=false",
-                           "-shared", "-Xcompiler", "-fPIC", "-I", CSRC, "-o", str(lib), str(src)])
+                           "-shared", "-Xcompiler", "-fPIC", "-I", CSRC, "-o", str(d / "libr.so"), str(d / "r.cu")])
+    return ctypes.CDLL(str(d / "libr.so"))
+
+
+@pytest.mark.gpu
+def test_equal_to_the_operators(lib):
     x, a = operands()
     out = (ctypes.c_ulonglong * 5)()
-    f = ctypes.CDLL(str(lib)).run
+    f = lib.run
     f.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_longlong, ctypes.c_void_p]
     assert f(x.ctypes.data, a.ctypes.data, x.size, ctypes.byref(out)) == 0
     assert list(out)[:4] == [0, 0, 0, 0]      # roots, reciprocals, refined ones, quotients
     assert 0 < out[4] < 1000                  # the exception is met and is rare
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("span", [0.01, 1.5, np.log(1e9)])
+def test_power(lib, span):
+    """Each rounding is at most 2^-53 of its value: u carries two and enters
+    five times, its powers and x^2 carry seven with their weights (6 in sum), a
+    tenth of which reaches the result, and one more: 1 + (10 + 6) / 10."""
+    x = np.exp(np.random.default_rng(3).uniform(-span, span, 1 << 21))
+    y = np.empty_like(x)
+    f = lib.pow_run
+    f.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_longlong]
+    assert f(x.ctypes.data, y.ctypes.data, x.size) == 0
+    want = x.astype(np.longdouble) ** np.longdouble(-0.7)
+    err = np.abs((y.astype(np.longdouble) - want) / want) * 2.0**53
+    print("x^-0.7: mean %.3f, max %.3f x 2^-53" % (err.mean(), err.max()))
+    assert err.max() <= 2.6
