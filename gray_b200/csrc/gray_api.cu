@@ -553,7 +553,8 @@ run_mixed(gray_ctx *c, Render *r, double t_init, double dt_dump, long long n_dum
 		if(!grid_ready(c))
 			return GRAY_ESTATE;
 		CK(launch_dyst_mixed_table(T, c->grid->gp, r->p.n_freq, r->d_queue, r->d_steps,
-		                           c->stream, c->mixed, dyst_between(c->grid->gp, &m, 1),
+		                           c->stream, c->mixed,
+		                           dyst_between(c->grid->gp, &m, 1, t_init - r->desc.t_init),
 		                           r->d_steps + 1));
 	} else {
 		CK(launch_mixed_table(T, r->p.n_freq, r->d_queue, r->d_steps, c->stream, c->mixed, &m));
