@@ -446,6 +446,10 @@ enter_cell(const GridParams &g, const DystConst &dc, Axis &A, Cell<RT> &C, int l
 			const float mg = 1e-5f * (fabsf(lo) + fabsf(hi));
 			A.xa = i0 == 2 ? hi + mg : i0 == 3 ? lo + mg : -INFINITY;
 			A.xb = i0 == 1 ? (g.single ? INFINITY : lo) : i0 == 3 ? hi - mg : INFINITY;
+			/* a level that holds alone: no factor, which may be above 1 and
+			 * would then send every stage here */
+			if(LV == 1)
+				A.inv = 0.0f;
 			if(LV == 2 && !g.physics) {
 				A.xa = -INFINITY;
 				A.xb = INFINITY;
