@@ -968,7 +968,10 @@ launch_dyst(const MixedTable &T, const GridParams &g, const DystConst &dc, int n
 		&occ, dyst_mixed_kernel<LV, FPL>, block, 0);
 	if(e != cudaSuccess)
 		return e;
+	/* a plan's blocks may be larger: as many warps per SM in these */
 	int per_sm = cfg.blocks_per_sm;
+	if(cfg.block > DYST_BLOCK)
+		per_sm *= (cfg.block + DYST_BLOCK - 1) / DYST_BLOCK;
 	if(per_sm <= 0 || per_sm > occ)
 		per_sm = occ > 0 ? occ : 1;
 	const long long want = (long long)per_sm * sms;

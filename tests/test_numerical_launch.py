@@ -82,3 +82,20 @@ def test_rays_past_the_levels_keep_their_cells(ctx, nu):
         assert np.linalg.norm(out[1][row] - out[0][row]) <= 1e-4 * np.linalg.norm(out[0][:8])
     grid(ctx, 64, -1.0, -1.0)
     assert past <= 1.2 * ms(ctx, cfg)
+
+
+@pytest.mark.gpu
+def test_plan_blocks_keep_their_warps(ctx):
+    """A plan of one 256-thread block per SM is eight warps in this kernel's
+    128-thread blocks too (four took 1.6 times as long)."""
+    grid(ctx, 64, 0.0, 0.0)
+    cfg = dict(BASE, n_width=300, n_height=200, dt_dump=-2.0, n_dump=5)
+    old = ctx.get_plan()
+    try:
+        ctx.set_plan(128, 2, 1)
+        two = ms(ctx, cfg)
+        ctx.set_plan(256, 1, 1)
+        one = ms(ctx, cfg)
+    finally:
+        ctx.set_plan(old.block, old.blocks_per_sm, old.rays_per_thread, old.rk4_rolled)
+    assert one <= 1.2 * two, (one, two)
