@@ -71,9 +71,8 @@ struct gray_ctx {
 	std::map<int, Render *> renders;
 	int next_id = 1;
 	Grid *grid = nullptr;
-	/* default plan (GRAY_PLAN_ESTIMATE): one ray per thread, 256-thread
-	 * blocks -- the shape the measuring planner picks on B200 for the
-	 * analytic torus renders */
+	/* default plan (GRAY_PLAN_ESTIMATE): one ray per thread, blocks of at
+	 * most 256 threads (the launches cut them to the kernel and the rays) */
 	MixedLaunch mixed = {256, 0, 0, 1};
 	std::map<int, Batch *> batches;
 	int next_batch = 1;

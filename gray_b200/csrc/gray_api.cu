@@ -1364,9 +1364,11 @@ gray_get_plan(const gray_ctx *c, gray_launch_plan *p)
 }
 
 /* Candidates: rays per thread {2, 1} x block {64, 128(, 256)} x blocks per
- * SM {all that fit, half of them} x RK4 stages {unrolled, looped}.  Each is timed (best of two) over the
- * first two dump intervals of every render in the batch, launched directly
- * (not through the graph). */
+ * SM {all that fit, half of them} x RK4 stages {unrolled, looped}.  Each is
+ * timed (best of two) over the first two dump intervals of every render in the
+ * batch, launched directly (not through the graph).  The unrolled one-ray
+ * kernel of a single render runs in 128 threads at most, so there 256 would
+ * time that shape a second time under a name it is never launched by. */
 extern "C" int
 gray_plan(gray_ctx *c, int id, int flags, gray_launch_plan *best)
 {
@@ -1377,8 +1379,9 @@ gray_plan(gray_ctx *c, int id, int flags, gray_launch_plan *best)
 		return GRAY_EINVAL;
 	CK(cudaSetDevice(c->device));
 	if(flags == GRAY_PLAN_ESTIMATE || b->spacetime == GRAY_ST_NUMERICAL) {
-		/* the rule: 256 threads, one ray each (the numerical kernel has
-		 * only this shape) */
+		/* the rule: 256 threads, one ray each; the launches make the blocks
+		 * smaller where that suits the kernel or the number of rays (the
+		 * numerical kernel's have 128 threads at most) */
 		c->mixed = MixedLaunch{256, 0, c->sms, 1, 0};
 		return gray_get_plan(c, best);
 	}
@@ -1398,7 +1401,8 @@ gray_plan(gray_ctx *c, int id, int flags, gray_launch_plan *best)
 	int nc = 0;
 	for(int rolled = 0; rolled <= 1; ++rolled)
 		for(int rpt = 2; rpt >= 1; --rpt)
-			for(int blk = 64; blk <= (rpt == 2 ? 128 : 256); blk *= 2) {
+			for(int blk = 64; blk <= (rpt == 2 || (trial.size() == 1 && !rolled) ? 128 : 256);
+			    blk *= 2) {
 				MixedLaunch m = {blk, 0, c->sms, rpt, rolled};
 				int occ = 0;
 				if(mixed_occupancy(b->n_freq, m, &occ) != cudaSuccess || occ <= 0)

@@ -220,10 +220,12 @@ int gray_batch_destroy(gray_ctx *ctx, int batch_id);
 int gray_batch_run(gray_ctx *ctx, int batch_id, double *ns);
 int gray_batch_steps(gray_ctx *ctx, int batch_id, uint64_t *steps);
 
-/* Launch shape of the persistent kernels. */
+/* Launch shape of the persistent kernels.  They make the blocks smaller than
+ * planned, and as many more of them, where one render or the numerical kernel
+ * wants 128 threads at most, and where few rays are spread over every SM. */
 typedef struct gray_launch_plan {
-	int32_t block;            /* threads per block                          */
-	int32_t blocks_per_sm;    /* 0 = as many as fit                         */
+	int32_t block;            /* threads per block, at most                 */
+	int32_t blocks_per_sm;    /* of that size; 0 = as many as fit           */
 	int32_t rays_per_thread;  /* 1 (scalar FP32) or 2 (packed f32x2)         */
 	int32_t rk4_rolled;       /* 0: the four RK4 stages unrolled (one RHS
 	                             body each), 1: one RHS body in a loop     */
