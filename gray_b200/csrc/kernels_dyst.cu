@@ -708,13 +708,13 @@ transfer(const MixedRender &c, int nf, unsigned gmask, int lane, double hs, floa
 		}
 }
 
-constexpr int DYST_BLOCK = 128;
+constexpr int DYST_BLOCK = 128, DYST_PER_SM = 3;
 
 /* LV: the time levels a ray's lanes hold; FPL: frequencies
  * per lane (0: geodesics alone).  The transfer pairs (I, tau) are FP64 and
  * ride along in the same RK4 stages. */
 template <int LV, int FPL>
-__global__ void __launch_bounds__(DYST_BLOCK, 3)
+__global__ void __launch_bounds__(DYST_BLOCK, DYST_PER_SM)
 dyst_mixed_kernel(const MixedTable T, const __grid_constant__ GridParams g, const DystConst dc,
                   const int nf, unsigned int *__restrict__ queue,
                   unsigned long long *__restrict__ steps, unsigned long long *__restrict__ inbox)
@@ -1007,6 +1007,12 @@ dyst_between(const GridParams &g, const MixedRender *r, int n, double t0)
 			return true;
 	}
 	return false;
+}
+
+int
+dyst_rays_per_sm(bool between)
+{
+	return DYST_BLOCK * DYST_PER_SM / (between ? 8 : 4);
 }
 
 cudaError_t

@@ -79,6 +79,8 @@ cudaError_t launch_mixed_table(const MixedTable &T, int n_freq, unsigned int *qu
  * the same n_freq; between: dyst_between() of the renders; inbox (nullable)
  * accumulates the steps that interpolate the grid */
 bool dyst_between(const GridParams &g, const MixedRender *r, int n, double t0 = 0.0);
+/* rays of such a launch that one SM holds at once */
+int dyst_rays_per_sm(bool between);
 cudaError_t launch_dyst_mixed_table(const MixedTable &T, const GridParams &g, int n_freq,
                                     unsigned int *queue, unsigned long long *steps,
                                     cudaStream_t st, const MixedLaunch &cfg, bool between,

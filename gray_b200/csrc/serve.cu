@@ -108,12 +108,12 @@ struct Request {
  * its steps per interval times the longer of one ray's step latency (a
  * small render's rays each run alone in a warp) and its rays' share of the
  * device's throughput.  The figures are B200 measurements of the mixed
- * kernels (analytic, numerical); they only size windows and never change a
- * result. */
-constexpr double STEP_LATENCY_S[2] = {1.5e-6, 0.75e-6};
-constexpr double STEP_COST_S[2] = {1.0 / 4.5e10, 1.0 / 4e10};
-/* rays of the numerical kernel an SM holds at once: 12 warps of 8 */
-constexpr unsigned NUM_RAYS_PER_SM = 96;
+ * kernels: a lone warp's analytic step takes 0.28-0.51 us (0 to 8 frequencies,
+ * 0.46 at 4 frequencies 60 M out) and 5.4e10 a second fill the device; a
+ * numerical geodesic's 1.04 us inside the box, and 3.9e10 a second over a path
+ * through it.  They only size windows and never change a result. */
+constexpr double STEP_LATENCY_S[2] = {0.46e-6, 1.04e-6};
+constexpr double STEP_COST_S[2] = {1.0 / 5.4e10, 1.0 / 3.9e10};
 constexpr double MIN_ITER_S = 0.05;
 
 /* steps of one ray per interval: the analytic cap |dt|/n_sub
@@ -251,19 +251,23 @@ release(Server *S, Request *r)
  * time on their two streams.  Each launch sizes its grid to its SM count,
  * so with both kinds in flight neither grid takes the whole device and the
  * other kind's launch does not wait for it to drain.  While the numerical
- * renders' rays fit on at most half the SMs at once, they get the SMs that hold them all: their windows were sized for
- * rays that run at once.  Otherwise the SMs are split by the kinds'
- * estimated work this iteration. */
+ * renders' rays fit on at most half the SMs at once (half as many per SM where
+ * they run between the time levels), they get the SMs that hold them all:
+ * their windows were sized for rays that run at once.  Otherwise the SMs are
+ * split by the kinds' estimated work this iteration. */
 void
-split_sms(const Server *S, const unsigned long long *total, int *ana_sms, int *num_sms)
+split_sms(const Server *S, const unsigned long long *total, const bool *between, int *ana_sms,
+          int *num_sms)
 {
 	const int sms = S->c->sms;
 	double work[2] = {0.0, 0.0};
 	for(const Request *r : S->inflight)
 		work[r->p.spacetime == GRAY_ST_NUMERICAL ? 1 : 0] += r->window * interval_s(r);
 	unsigned long long need = 0; /* SMs */
-	for(int g = NUM_GROUP; g < GROUPS; ++g)
-		need += (total[g] + NUM_RAYS_PER_SM - 1) / NUM_RAYS_PER_SM;
+	for(int g = NUM_GROUP; g < GROUPS; ++g) {
+		const unsigned per = (unsigned)dyst_rays_per_sm(between[g]);
+		need += (total[g] + per - 1) / per;
+	}
 	*ana_sms = *num_sms = sms;
 	if(work[0] <= 0.0 || work[1] <= 0.0 || sms < 2)
 		return;
@@ -376,7 +380,10 @@ iterate(Server *S, std::vector<Request *> &fresh)
 	MixedLaunch cfg = c->mixed;
 	cfg.sms = c->sms;
 	int num_sms = c->sms;
-	split_sms(S, total, &cfg.sms, &num_sms);
+	bool between[GROUPS] = {false};
+	for(int g = NUM_GROUP; g < GROUPS; ++g)
+		between[g] = count[g] && dyst_between(c->grid->gp, &S->h_tab[start[g]], count[g]);
+	split_sms(S, total, between, &cfg.sms, &num_sms);
 	for(int g = 0; g < GROUPS; ++g) {
 		if(!count[g])
 			continue;
@@ -391,8 +398,7 @@ iterate(Server *S, std::vector<Request *> &fresh)
 			dc.block = 256;
 			dc.sms = num_sms;
 			e = launch_dyst_mixed_table(T, c->grid->gp, g - NUM_GROUP, q, S->d_steps + g,
-			                            S->s[1], dc,
-			                            dyst_between(c->grid->gp, &S->h_tab[start[g]], count[g]));
+			                            S->s[1], dc, between[g]);
 		} else {
 			e = launch_mixed_table(T, g, q, S->d_steps + g, S->s[0], cfg,
 			                       count[g] == 1 ? &S->h_tab[start[g]] : nullptr);
