@@ -339,9 +339,8 @@ template <int LV>
 __device__ __forceinline__ int
 level_code(const GridParams &g, float ft)
 {
-	if(LV == 2 && !g.physics)
-		return ft == ft ? 3 : 0;
-	return g.single ? 1 : (ft < 1.0f ? 1 : 0) | (ft > 0.0f ? 2 : 0);
+	const int both = LV == 2 && !g.physics ? 3 : 0;
+	return g.single ? 1 : (ft < 1.0f ? 1 | both : 0) | (ft > 0.0f ? 2 | both : 0);
 }
 
 template <bool RT>
@@ -443,17 +442,13 @@ enter_cell(const GridParams &g, const DystConst &dc, Axis &A, Cell<RT> &C, int l
 			}
 			i0 = level_code<LV>(g, w);
 			/* times at which the rounded factor surely gives the same code */
-			const float mg = 1e-5f * (fabsf(lo) + fabsf(hi));
+			const float mg = LV == 2 && !g.physics ? -INFINITY : 1e-5f * (fabsf(lo) + fabsf(hi));
 			A.xa = i0 == 2 ? hi + mg : i0 == 3 ? lo + mg : -INFINITY;
 			A.xb = i0 == 1 ? (g.single ? INFINITY : lo) : i0 == 3 ? hi - mg : INFINITY;
 			/* a level that holds alone: no factor, which may be above 1 and
 			 * would then send every stage here */
 			if(LV == 1)
 				A.inv = 0.0f;
-			if(LV == 2 && !g.physics) {
-				A.xa = -INFINITY;
-				A.xb = INFINITY;
-			}
 			if(i0 == 0 || (LV == 1 && i0 == 3))
 				A.xa = INFINITY;
 		} else {
