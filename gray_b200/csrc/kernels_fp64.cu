@@ -251,13 +251,14 @@ __device__ __forceinline__ bool
 torus_rt64(const RenderParams &p, bool ok, const double *s, const Aux64 &x, double *ds)
 {
 	bool emits = false;
-	double shift = 1.0, irs = 0.0;
+	double shift = 1.0, n = 0.0, pw = 0.0, is2 = 0.0, ish = 0.0;
 	if(x.r > p.risco && p.flow == GRAY_FLOW_TORUS) {
 		const double q1 = s[1], q2 = s[2];
 		const double kt = x.flu - s[4];
 		const double kx = fma(x.flu, x.lx, s[5]);
 		const double ky = fma(x.flu, x.ly, s[6]);
 		const double R2 = fma(q1, q1, q2 * q2);
+		double irs;
 		const double sr = sqrt_rn(x.r, irs);
 		const double Om = rcp_fast(fma(x.r, sr, p.a));
 		const double vv = fma(Om * Om, R2, -1.0);
@@ -268,14 +269,14 @@ torus_rt64(const RenderParams &p, bool ok, const double *s, const Aux64 &x, doub
 		shift = -utf * fma(Om, fma(q1, ky, -(q2 * kx)), kt);
 		emits = D > 0.0 && !(shift <= 0.0);
 		ok = ok && (!emits || (D > 1e-30 && shift > 1e-9 && shift < 1e9));
-	}
-	double n = 0.0;
-	if(emits) {
+		pw = pow_m07(shift);
+		is2 = rcp_fast(fma(shift, shift, GRAY_EPSILON));
+		ish = rcp_fast(shift);
 		const double v = div_rn(s[3], x.r, x.ir), v2 = v * v;
 		const double w = x.ir * irs, wl = fma(x.ir, irs, -w);
 		const double g = fma(v2, p.torus_ig, v2 * p.torus_igl);
 		n = fma(w, p.torus_n15, fma(w, p.torus_n15l, wl * p.torus_n15)) * exp(-g);
-		emits = n != 0.0;
+		emits = emits && n != 0.0;
 	}
 	if(!emits || !ok) {
 #pragma unroll
@@ -283,9 +284,8 @@ torus_rt64(const RenderParams &p, bool ok, const double *s, const Aux64 &x, doub
 			ds[8 + i] = 0.0;
 		return ok;
 	}
-	const double tfac = (p.torus_kappa * n) * rcp_fast(shift);
-	const double is2  = rcp_fast(fma(shift, shift, GRAY_EPSILON));
-	const double jfac = (n * is2) * pow_m07(shift);
+	const double tfac = (p.torus_kappa * n) * ish;
+	const double jfac = (n * is2) * pw;
 #pragma unroll
 	for(int i = 0; i < NF; ++i) {
 		ds[8 + i]      = -((jfac * p.nupow[i]) * exp(-s[8 + NF + i]));
