@@ -56,8 +56,8 @@ METRIC = "ray-steps/s"
 
 # DRAM bytes (read + write) of one full-size launch of the dominant kernel,
 # from one-pass ncu captures (dram__bytes_read.sum + dram__bytes_write.sum).
-TRAFFIC = {"torus_rt_1024": 149105664 + 127566848,
-           "numerical_128": 500394240 + 17862656}
+TRAFFIC = {"torus_rt_1024": 147723520 + 126620416,
+           "numerical_128": 394353152 + 16503040}
 # Host-to-device bytes of one render through the C ABI: the render's table
 # entry (sizeof(MixedRender) in gray_b200/csrc/mixed_table.h), which the
 # analytic kernel's one-render launch also carries as its kernel parameter;

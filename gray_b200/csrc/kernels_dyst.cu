@@ -2,8 +2,12 @@
  * Mixed-precision persistent kernel for numerical spacetimes (interp.cl +
  * dyst.cl): several lanes per ray, the ray's cell held in registers.
  *
- * A ray moves about 0.01 M per stage through cells 0.2-2 M wide, so the same
- * 8 corners serve dozens to hundreds of RHS evaluations.  Lane m of a ray's
+ * A ray moves at most 0.01 M per stage through cells of up to 2 M, so the same
+ * 8 corners mostly serve dozens to hundreds of RHS evaluations.  (The fisheye
+ * nodes crowd at the coordinate planes: at 256^3 cells are thinner than a
+ * stage's 0.01 M within 0.13 M of one.  A ray that runs along a plane searches
+ * and reads at every RHS, and its warp waits; it is a thin part of an image.)
+ * Lane m of a ray's
  * four lanes owns x^m, u^m and row m of the Christoffel symbols: the ten
  * Gamma^m_ab of the cell's 8 corners stay in 80 of its registers and are
  * read from memory only when the ray enters another cell.  An RHS is then 40
@@ -12,9 +16,10 @@
  * fit no thread, so every RHS fetched 1,280 bytes per ray through L1, and
  * that latency bound the kernel.
  *
- * What bounds it: the FP32 pipe and issue, about evenly (FMA pipe 56% of its
- * cycles, issue 63%, 158 instructions per warp and RHS against 105 counted
- * from the algorithm; 12 warps per SM at 168 registers).  Measured, B200 at
+ * What bounds it: the FP32 pipe and issue, about evenly (512^2 rays inside the
+ * box: FMA pipe 57% of its cycles, issue 60%, 141 instructions per warp and
+ * RHS against 105 counted from the algorithm; 12 warps per SM at 168
+ * registers).  Measured, B200 at
  * 1965 MHz, one ray per thread before and four lanes now: 512^2 rays at 200 M
  * on a 128^3 grid 530 -> 197 ms (1.48e10 -> 3.99e10 ray-steps/s), 97 x 72
  * rays on a 256^3 grid 243 -> 22.8 ms, 160 x 120 rays between two levels
@@ -34,7 +39,8 @@
  * e^-tau chains the stages, through one shuffle.  With a frequency per lane
  * instead, 200 x 160 rays between two levels took 28.1 ms for one frequency
  * (now 19.0) and 160 x 120 rays 17.5 ms for four (14.3); eight frequencies in
- * one level, where no lane idled, 14.7 (18.0).
+ * one level, where no lane idled, 14.7 (18.0).  At 168 registers these forms
+ * spill (244 to 310 bytes of stores).
  *
  * Grid layout: per time level float [nz][ny][nx][GRAY_NSTRIDE] with the
  * fields of one grid point contiguous (Gamma 0..39, g 40..49, rho 50, pad).

@@ -494,15 +494,16 @@ icond64_kernel(const RenderParams p, double *__restrict__ data,
  * itself: launched one by one, every interval waited for the rays that take
  * 10^4 short steps to the horizon in one of them.
  *
- * What bounds it: the FP64 pipe (78% of its rate without transfer at 512 x
- * 384 rays), and where few rays run, or few are left, the latency of a step:
- * 1.55 us alone, of dependent FP64 operations.  Measured before (the
- * operators, one launch per interval) and now, B200 at 1965 MHz: 251 x 190
- * rays through the hole's region, 4 frequencies, 172.0 -> 87.3 ms, 1
- * frequency 127.3 -> 75.0; 512 x 384 rays over one interval, 4 frequencies,
- * 46.9 -> 29.9 ms, none 12.4 -> 11.2; 24 x 16 rays 39.1 -> 26.0.  With 168
- * registers for 12 warps per SM instead of 8 the 512 x 384 render takes 27.6
- * ms, but the rays that end last step slower: 94.3 ms at 251 x 190. */
+ * What bounds it: the FP64 pipe (82% of its rate without transfer and 70% with
+ * four frequencies at 512 x 384 rays), and where few rays run, or few are left,
+ * the latency of a step: 1.33 us alone (3.28 where four frequencies emit), of
+ * dependent FP64 operations.  Measured with the operators and one launch per
+ * interval, and now, B200 at 1965 MHz: 160 x 120 rays through the hole's
+ * region, 4 frequencies, 126.3 -> 58.1 ms, 1 frequency 123.2 -> 51.1, none
+ * 97.2 -> 40.2; 512 x 384 rays over one interval, 4 frequencies, 46.9 -> 25.0,
+ * none 12.4 -> 11.0; 24 x 16 rays 40.2 -> 23.1.
+ * One warp more per scheduler (168 registers) gained 8% on the 512 x 384
+ * render, but the rays that end last step slower: 251 x 190 rays lost 8%. */
 template <int NF>
 __global__ void __launch_bounds__(EVOLVE64_BLOCK)
 evolve64_kernel(const __grid_constant__ RenderParams p, double *__restrict__ data,

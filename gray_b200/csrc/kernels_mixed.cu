@@ -683,6 +683,8 @@ ticks(const SlotView<UNI> &v, int k, const V *hi, const V *lo)
  * rays 0.576 -> 0.407, 512 x 384 rays 4.32 -> 3.94, 1024^2 rays through the
  * hole's region 226.8 -> 212.3 (bit-identical).  What is left of a lone
  * warp's step is the dependent FP32 chain of its four RHS. */
+/* Neither matters much: 4 or 16 for the first and 16 or 64 for the second
+ * measured within 0.6% of these on six renders from 24 x 16 to 1024^2 rays. */
 constexpr int FAR_MIN = 8;      /* fewer are not worth the question         */
 constexpr int COAST_RETRY = 32; /* ordinary steps before it is asked again  */
 
@@ -1122,10 +1124,11 @@ launch_nf(const MixedTable &T, const MixedRender &R1, unsigned int *queue,
 	if(block > maxb || block % 32)
 		return cudaErrorInvalidValue;
 	/* few rays: smaller blocks, down to one warp, until every SM has a warp
-	 * and every scheduler one before any has two.  A lone warp's step takes
-	 * 1,260 cycles of dependent latency, and two on one scheduler half as
-	 * long again while others idle: 64^2 rays with 4 frequencies took
-	 * 62.9 ms in 256-thread blocks and take 45.8 ms */
+	 * and every scheduler one before any has two.  A lone warp's step is one
+	 * chain of dependent latency (800 to 900 cycles at 4 frequencies), and two
+	 * on one scheduler take half as long again while others idle: 64^2 rays
+	 * with 4 frequencies took 62.9 ms in 256-thread blocks and 45.8 ms so,
+	 * when a step was 1,260 cycles */
 	const int sms = cfg.sms > 0 ? cfg.sms : 148;
 	const unsigned long long warps = (T.total + 32 * Lanes<V>::N - 1) / (32 * Lanes<V>::N);
 	if(warps < (unsigned long long)sms * (block / 32))

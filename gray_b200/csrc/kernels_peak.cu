@@ -72,7 +72,7 @@ fma64_kernel(double *out, int iters, double a, double b)
 		out[0] = s;
 }
 
-/* L1 load bandwidth with the numerical kernel's load instruction: 32-byte
+/* L1 load bandwidth with the widest load instruction: 32-byte
  * loads (ld.global.nc.v8.f32) from a 16 KiB window that stays resident in
  * L1, a warp's 32 lanes reading 32 consecutive rows (1 KiB, fully used
  * lines), so that the L1 data path, not its tag lookups, is the limit: the
