@@ -471,7 +471,7 @@ def ours_arm(args, cfg, rank, local_rank, world, dist):
                 "roofline": {"bound": "fp64", "achieved": a64, "peak": peak64 / 1e12,
                              "unit": "TFLOP/s", "frac": a64 * 1e12 / peak64,
                              "flop_per_ray_step": flops.fp64_per_step(nf)},
-                "launches_per_render": 1 + int(cfg["n_dump"])}
+                "launches_per_render": 2}
 
     # ---- end to end: render + device-to-host copy of the state, host buffers
     host = torch.empty((8 + 2 * nf) * n_rays, dtype=torch.float64, pin_memory=True).numpy()

@@ -107,13 +107,17 @@ struct Request {
 /* Estimated seconds of one dump interval of a render on the shared device:
  * its steps per interval times the longer of one ray's step latency (a
  * small render's rays each run alone in a warp) and its rays' share of the
- * device's throughput.  The figures are B200 measurements of the mixed
- * kernels: a lone warp's analytic step takes 0.28-0.51 us (0 to 8 frequencies,
- * 0.46 at 4 frequencies 60 M out) and 5.4e10 a second fill the device; a
- * numerical geodesic's 1.04 us inside the box, and 3.9e10 a second over a path
- * through it.  They only size windows and never change a result. */
-constexpr double STEP_LATENCY_S[2] = {0.46e-6, 1.04e-6};
-constexpr double STEP_COST_S[2] = {1.0 / 5.4e10, 1.0 / 3.9e10};
+ * device's throughput (analytic, numerical).  The figures size windows and
+ * never change a result.  The costs are the mixed kernels' rates on a B200 less
+ * a margin (5.4e10 and 3.9e10 steps/s).  The analytic latency is three times a
+ * lone warp's capped step (0.46 us at 4 frequencies), because an interval near
+ * the horizon takes many more steps than n_sub; the numerical one is below a
+ * step's 1.04 us inside the box, because outside it steps run in chunks.  With
+ * the bare measurements in their place windows outlast their estimate, and the
+ * default serving sweep's median latency at 1.0/s rose from 0.17 to 0.19 s (its
+ * slowdown p99 fell from 2.6 to 2.5). */
+constexpr double STEP_LATENCY_S[2] = {1.5e-6, 0.75e-6};
+constexpr double STEP_COST_S[2] = {1.0 / 4.5e10, 1.0 / 4e10};
 constexpr double MIN_ITER_S = 0.05;
 
 /* steps of one ray per interval: the analytic cap |dt|/n_sub
